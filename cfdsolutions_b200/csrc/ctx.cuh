@@ -80,43 +80,29 @@ struct Levels {
     int max_width = 0;
 };
 
-// Factors of one storage type in the triangular solves' packed layout
-// (lower slots, upper slots, inverted diagonal blocks; see k_mc_pack).
-template <typename TM>
-struct McPack {
-    DevBuf<TM> L, U, D;
-};
-
 // Block multicolour ordering of the ILU(0) preconditioner (ilu_mc.cu): rows
 // are grouped in patches of consecutive rows, the patch graph is coloured
 // (DSATUR), and the factorisation order is colour by colour, row index within
 // a colour.
 struct Abmc {
     bool built = false;
-    int ncolor = 0, maxrow = 0, maxlev = 0, maxstage = 0;
+    int ncolor = 0, maxrow = 0, maxstage = 0;
     std::vector<int> cptr;            // host [ncolor+1] into patches
     std::vector<int> h_pcolor;        // host colour of each patch
     DevBuf<int> patches;              // patch ids in colour order
     DevBuf<int> slot;                 // [nnzb] per row: lower slots (factorisation order) | diag | upper slots
-    DevBuf<int> scol;                 // [nnzb] column of each slot entry
-    DevBuf<int4> meta;                // per row: external lower, lower, intra-patch upper, lev_f | lev_b << 16
-    DevBuf<int2> plev;                // per patch: last forward level, last backward level
-    DevBuf<int4> hdr;                 // [nnzb] per lower block: slot of inv(U_pp), pairs, local slot
+    DevBuf<int4> meta;                // per row: external lower, lower, intra-patch upper, 0
+    DevBuf<unsigned> loc;             // [nnzb] place of each slot entry's factor block in M
+    int64_t nelem = 0;                // elements of M
+    DevBuf<int4> hdr;                 // [nnzb] per lower block: place of inv(U_pp) in M, pairs, local slot
     DevBuf<int64_t> pair_ptr;         // [n+1] update pairs of each row
-    DevBuf<int2> pairs;               // (slot of U_pj, local slot of (i,j))
-    // triangular solves: per row in launch order (colour, patch position, row)
-    DevBuf<int4> rowf;                // {row, off-patch lower slots, lower slots, first lower slot in M}
-    DevBuf<int4> rowb;                // {row, intra-patch upper slots, upper slots, diagonal slot in M}
-    DevBuf<int4> rowl;                // {forward level, patch's last, backward level, patch's last}
-    // packed layout: per patch position its first lower / upper slot row
-    // (slots of 32 rows x 25 entries), and each slot's column per row
-    int64_t nlslot = 0, nuslot = 0;
-    DevBuf<int64_t> lslot, uslot;     // [npatch+1]
-    DevBuf<int> colL, colU;           // [slots][32]
-    McPack<float> pk32;
-    McPack<double> pk64;
-    template <typename TM>
-    McPack<TM> &pack();
+    DevBuf<int2> pairs;               // (place of U_pj in M, local slot of (i,j))
+    // triangular solves (0 forward, 1 backward), patches in launch order: per
+    // patch {first 16-byte word of its lists, words, first unit of its region
+    // of M, units}; per colour the largest {words, units, columns, elements before the slots}
+    DevBuf<int4> desc[2];
+    DevBuf<uint4> lists[2];
+    std::vector<int4> shape[2];
     // captured applies (one CUDA graph per factor / input / scratch / output
     // pointer set; the GMRES driver reuses a few such sets)
     struct Graph {
@@ -130,11 +116,6 @@ struct Abmc {
     }
     ~Abmc() { clear_graphs(); }
 };
-template <>
-inline McPack<float> &Abmc::pack<float>() { return pk32; }
-template <>
-inline McPack<double> &Abmc::pack<double>() { return pk64; }
-
 // Plan of the pipelined residual step (cfd_residual_step with host buffers):
 // node chunks, their dependencies through the node graph's bandwidth, the
 // boundary edges and boundary nodes of each chunk, and the copy streams.

@@ -9,19 +9,20 @@
 // coloured by DSATUR.  The factorisation order is: colours in increasing
 // order, rows of a colour in increasing index.  Two patches of one colour are
 // never coupled, so every patch of a colour is factored (or solved) by its own
-// CTA in one launch per colour; inside a patch the rows follow their local
-// dependency levels, separated by __syncthreads().  This is ILU(0) of P A P^T
+// warp or CTA in one launch per colour.  This is ILU(0) of P A P^T
 // for the permutation P of that order (the ordering idea is the algebraic block
 // multicolour ordering of Iwashita, Nakashima and Takahashi, IPDPS 2012).
 //
 // Storage: `slot` lists each row's CRS slots as [lower, in factorisation
-// order | diagonal | upper, in factorisation order]; the factors are stored
-// in that order (entry u of row i at block IA[i] + u): L (unit diagonal) for
-// the lower entries, inv(U_ii) for the diagonal, U for the upper entries.
+// order | diagonal | upper, in factorisation order]; `loc` is the place of
+// entry u of row i (at IA[i] + u) in M: L (unit diagonal) for the lower
+// entries, inv(U_ii) for the diagonal, U for the upper entries.
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdint>
+#include <cstring>
 #include <set>
 #include <tuple>
 #include <vector>
@@ -95,6 +96,33 @@ __device__ __forceinline__ bool warp_inverse5(double &a, double &v, int lane) {
     return ok;
 }
 
+// Triangular solves: six warps per patch, six groups of five lanes per warp
+// (lanes 30 and 31 idle), a group per row.
+constexpr int kMcWarps = 6, kMcGroups = 6 * kMcWarps, kMcSolveThreads = 32 * kMcWarps;
+static_assert(kMcGroups >= kMcRows, "a group per row");
+
+// Storage of the factors in M.  A patch's lower blocks are one region, its
+// inverted diagonal and upper blocks another, so that one triangular solve of
+// a patch reads one contiguous run.  A region holds [diagonal blocks, by row
+// | blocks inside the patch, by row | slots of off-patch blocks]: slot t of
+// warp w holds the t-th off-patch block of each of the warp's six rows.
+// Rows are given to groups by decreasing number of off-patch blocks, so a
+// warp's six rows have nearly equal numbers and few places stay empty (8 % of
+// M on the tet cubes; they hold zeros).  Element 30 k + 5 g + c of a slot is
+// entry (row (k + c) mod 5, column c) of group g's block: lane c of a group
+// reads column c of its block with five loads, each of 30 consecutive values
+// per warp.  The other blocks are row-major.  A block's place is its first
+// element / 5, with kMcSlotBit for one in a slot.  Regions start at multiples
+// of 20 elements (16 bytes in FP32 and FP64).
+constexpr unsigned kMcSlotBit = 0x80000000u;
+constexpr int kMcSlot = 150, kMcUnit = 20;
+
+// Element (r, c) of the block at place p.
+__device__ __forceinline__ int64_t mc_element(unsigned p, int r, int c) {
+    const int k = (p & kMcSlotBit) ? 30 * (r >= c ? r - c : r - c + 5) : 5 * r;
+    return (int64_t)(p & ~kMcSlotBit) * 5 + k + c;
+}
+
 // Shared-memory bytes of one warp of k_mc_factor (factor blocks staged in
 // their storage type TM), rounded up to 16.
 template <typename TM>
@@ -114,14 +142,14 @@ __host__ __device__ inline size_t mc_factor_warp_bytes(int maxrow, int maxstage)
 // setup.  All those loads are issued together, then the elimination runs from
 // shared memory: for each lower block, in factorisation order,
 // L_ip = A_ip inv(U_pp) and A_ij -= L_ip U_pj over the row's pairs of p.
-// The factors are stored in each row's factorisation order (row i's entry u of
-// the slot list at M[(IA[i] + u) * 25]), so the solves read them as a stream.
-// hdr[IA[i]+u] = (M position of inv(U_pp), pairs, CRS-local slot of (i,p));
-// pairs are (M position of U_pj, CRS-local slot of (i,j)).
+// The factors are stored by patch, as the triangular solves stage them:
+// loc[IA[i]+u] is the place of row i's entry u.
+// hdr[IA[i]+u] = (place of inv(U_pp), pairs, CRS-local slot of (i,p));
+// pairs are (place of U_pj, CRS-local slot of (i,j)).
 template <typename TA, typename TM>
 __global__ void k_mc_factor(const int *__restrict__ patches, int npatch, int n, int maxrow, int maxstage,
                             const int *__restrict__ IA, const int *__restrict__ slot, const int4 *__restrict__ meta,
-                            const int4 *__restrict__ hdr,
+                            const int4 *__restrict__ hdr, const unsigned *__restrict__ loc,
                             const int64_t *__restrict__ pair_ptr, const int2 *__restrict__ pairs,
                             const TA *__restrict__ A, TM *__restrict__ M, int *__restrict__ err) {
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -133,7 +161,7 @@ __global__ void k_mc_factor(const int *__restrict__ patches, int npatch, int n, 
     double *w = reinterpret_cast<double *>(reg + (size_t)maxrow * sizeof(int4));  // [maxrow][25] row blocks
     TM *stg = reinterpret_cast<TM *>(w + (size_t)maxrow * 25);       // [maxstage][25] staged factor blocks
     int *pm = reinterpret_cast<int *>(stg + (size_t)maxstage * 25);  // [maxstage] CRS-local slot of each pair
-    int *src = pm + maxstage;                                         // [maxstage] M position of staged blocks
+    int *src = pm + maxstage;                                         // [maxstage] place of staged blocks in M
     int *sl = src + maxstage;                                         // [maxrow] CRS-local slot of list entry u
     const int pidx = blockIdx.x * nwarp + wid;
     if (pidx >= npatch) return;  // whole warp; no CTA barrier follows
@@ -167,9 +195,9 @@ __global__ void k_mc_factor(const int *__restrict__ patches, int npatch, int n, 
             __syncwarp();
             const int nst = nlo + npair;
             for (int t = lane; t < nst; t += 32) {
-                const TM *mb = M + (int64_t)src[t] * 25;
+                const unsigned p = (unsigned)src[t];
 #pragma unroll
-                for (int k = 0; k < 25; k++) stg[t * 25 + k] = mb[k];
+                for (int k = 0; k < 25; k++) stg[t * 25 + k] = M[mc_element(p, k / 5, k % 5)];
             }
             __syncwarp();
             int t0 = 0;
@@ -208,8 +236,8 @@ __global__ void k_mc_factor(const int *__restrict__ patches, int npatch, int n, 
             }
             __syncwarp();
             for (int e = lane; e < len * 25; e += 32) {
-                const int u = e / 25;
-                st<TM>(M + (int64_t)base * 25 + e, w[sl[u] * 25 + (e - 25 * u)]);
+                const int u = e / 25, rc = e - 25 * u;
+                st<TM>(M + mc_element(loc[base + u], rc / 5, rc % 5), w[sl[u] * 25 + rc]);
             }
             __syncwarp();
         }
@@ -225,246 +253,332 @@ __global__ void k_mc_factor(const int *__restrict__ patches, int npatch, int n, 
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// Resident CTAs per SM the triangular solves are compiled for: FP32 factors
-// fit 8 in 48 registers; FP64 factors keep 6 (64 registers), which measured
-// faster than 8 at 128^3 (2.69 against 2.88 ms per apply).
-template <typename TM>
-struct McMinBlocks {
-    static constexpr int value = sizeof(TM) == 8 ? 6 : 8;
+// 16-byte asynchronous copy global -> shared (LDGSTS), and the wait for all of
+// the thread's copies.
+__device__ __forceinline__ void copy16(void *smem, const void *gmem) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem)
+                 : "memory");
+}
+// Starts fetching [gmem, gmem + bytes) from DRAM into L2 (multiples of 16).
+__device__ __forceinline__ void prefetch_l2(const void *gmem, unsigned bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(gmem), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// A group's row in its patch (255 none) and its off-patch blocks.
+struct McGroup {
+    unsigned short row, next;
 };
+static_assert(sizeof(McGroup) == 4, "packed in the patch lists");
+// Byte offsets of a patch's lists: int4 {off-patch columns, steps, rows, first
+// row}, int4 {first element of the slots in the region, slots, 0, 0}, per
+// warp {first slot, slots}, the groups; then the distinct off-patch columns,
+// the steps (six operations each, see mc_op) and, 16 bits per slot and group,
+// its column's index among those columns (their number for an empty place).
+constexpr int kMcWarpAt = 32, kMcGroupAt = kMcWarpAt + 4 * kMcWarps, kMcColAt = kMcGroupAt + 4 * kMcGroups;
 
-// Blocks of a row inside its own patch staged in shared memory before the
-// level loop of a triangular solve (more go through the load path).
-template <typename TM>
-struct IntraCap {
-    static constexpr int K = sizeof(TM) == 8 ? 3 : 6;
-};
-
-// Off-patch blocks of a row whose columns a triangular solve fetches before
-// its dependency wait (the rest are read in its loop).
-constexpr int kMcPrefetch = 4;
-
-// Forward solve y = L^-1 r over the patches of one colour: five threads per
-// row (thread m forms component m).  Lower blocks in other patches belong to
-// earlier colours (complete in y) and are summed first; the row's blocks
-// inside the patch are staged in shared memory before the level loop, which
-// then only waits on shared memory.  CTA b takes the patch at position b of
-// the colour and reads the factors in the packed layout k_mc_pack writes:
-// slot t of every row of the patch side by side, so that for each (slot,
-// component) the CTA's 160 threads read 160 consecutive values (thread q*5+m
-// the entry (m, c) of row q's block) instead of five 32-byte sectors per row.
-// rowf / rowl hold the rows' records ({i, off-patch lower slots, lower slots}
-// and {level, last level of the patch, ..}; i = -1 past the mesh), L / cl the
-// patch's factors and columns (off-patch slots: global columns, intra-patch
-// slots: patch-local ones).  Everything constant is read before the wait;
-// after it one round trip fetches the earlier colours' y.
-template <typename TM>
-__global__ void __launch_bounds__(5 * kMcRows, McMinBlocks<TM>::value)
-    k_mc_fwd(const int4 *__restrict__ rowf, const int4 *__restrict__ rowl, const int64_t *__restrict__ lslot,
-             const int *__restrict__ colL, const TM *__restrict__ PL, const double *__restrict__ r,
-             double *__restrict__ y) {
-    constexpr int K = IntraCap<TM>::K, PF = kMcPrefetch;
-    constexpr int T = 5 * kMcRows;
-    __shared__ double ys[T];
-    __shared__ TM pa[K * 5][T];  // [t*5+c][thread]
-    __shared__ unsigned char pj[K][T];
-    const int tid = threadIdx.x;
-    const int q = tid / 5, m = tid - 5 * q;
-    const int4 rf = rowf[blockIdx.x * kMcRows + q];
-    const int4 rl = rowl[blockIdx.x * kMcRows + q];
-    const int64_t ls = lslot[blockIdx.x];
-    const TM *L = PL + ls * (25 * kMcRows) + tid;  // slot t, column c of the block: L[(t * 5 + c) * T]
-    const int *cl = colL + ls * kMcRows + q;       // column of slot t: cl[t * kMcRows]
-    const bool act = rf.x >= 0;
-    const int i = rf.x, nx = rf.y, nlo = rf.z, lev = rl.x;
-    double s = 0.0;
-    int col[PF];
-    // the next colour's launch may start staging its constant factors now
-    pdl_trigger();
-    if (act) {
-#pragma unroll
-        for (int t = 0; t < K; t++)
-            if (nx + t < nlo) {
-                pj[t][tid] = (unsigned char)cl[(nx + t) * kMcRows];
-#pragma unroll
-                for (int c = 0; c < 5; c++) pa[t * 5 + c][tid] = L[((nx + t) * 5 + c) * T];
-            }
-#pragma unroll
-        for (int t = 0; t < PF; t++) col[t] = t < nx ? cl[t * kMcRows] : 0;
-        // r is complete before the first colour's launch starts, so before this one's
-        s = r[(int64_t)i * 5 + m];
-    }
-    pdl_wait();  // the earlier colours' y are complete from here on
-    if (act) {
-#pragma unroll
-        for (int t = 0; t < PF; t++)
-            if (t < nx) {
-                const double *yv = y + (int64_t)col[t] * 5;
-#pragma unroll
-                for (int c = 0; c < 5; c++) s = fma(-ld<TM>(L + (t * 5 + c) * T), yv[c], s);
-            }
-#pragma unroll 4
-        for (int t = PF; t < nx; t++) {
-            const double *yv = y + (int64_t)cl[t * kMcRows] * 5;
-#pragma unroll
-            for (int c = 0; c < 5; c++) s = fma(-ld<TM>(L + (t * 5 + c) * T), yv[c], s);
-        }
-    }
-    const int last = rl.y;
-    for (int l = 0; l <= last; l++) {
-        if (act && lev == l) {
-#pragma unroll
-            for (int t = 0; t < K; t++)
-                if (nx + t < nlo) {
-                    const double *yv = ys + pj[t][tid] * 5;
-#pragma unroll
-                    for (int c = 0; c < 5; c++) s = fma(-(double)pa[t * 5 + c][tid], yv[c], s);
-                }
-            for (int t = nx + K; t < nlo; t++) {
-                const double *yv = ys + cl[t * kMcRows] * 5;
-#pragma unroll
-                for (int c = 0; c < 5; c++) s = fma(-ld<TM>(L + (t * 5 + c) * T), yv[c], s);
-            }
-            ys[tid] = s;
-        }
-        __syncthreads();
-    }
-    if (act) y[(int64_t)i * 5 + m] = s;
+// An operation of a step, on values v_r of the patch's rows: v_row -= block *
+// v_col for an intra-patch block or, diag, v_row = block * v_row with the
+// inverted diagonal block.  block counts from the region's start (diagonal
+// blocks first).  row = col = 32 for an idle group.
+__host__ __device__ inline unsigned mc_op(int block, int col, int row, bool diag) {
+    return (unsigned)block | ((unsigned)col << 10) | ((unsigned)row << 16) | (diag ? 0x80000000u : 0u);
 }
 
-// Backward solve z = U^-1 y over the patches of one colour (colours in
-// decreasing order): upper blocks in other patches belong to later colours.
-// rowb holds {i, intra-patch upper slots, upper slots, ..}; U / cu the
-// packed upper blocks (intra-patch slots first, patch-local columns) and D the
-// packed inverted diagonal blocks.  y is read after the wait: the last
-// forward colour may still be writing it when the first backward one starts.
+// Largest part of a region staged in shared memory, in units of kMcUnit
+// elements (the slots past it are read from global memory).  A colour whose
+// patches are all resident at once stages whole regions, for the shortest
+// patch (48^3, 340 patches per colour, FP64: 181 us per apply, 228 with 176
+// units); a larger one stages less, for more CTAs per SM (96^3, 2600 patches
+// per colour: FP64 795 us, 1005 with 640 units; FP32 521 and 568).
+constexpr int kMcStageUnits = 640;
 template <typename TM>
-__global__ void __launch_bounds__(5 * kMcRows, McMinBlocks<TM>::value)
-    k_mc_bwd(const int4 *__restrict__ rowb, const int4 *__restrict__ rowl, const int64_t *__restrict__ uslot,
-             const int *__restrict__ colU, const TM *__restrict__ PU, const TM *__restrict__ PD,
-             const double *__restrict__ y, double *__restrict__ z) {
-    constexpr int K = IntraCap<TM>::K, PF = kMcPrefetch;
-    constexpr int T = 5 * kMcRows;
-    __shared__ double zs[T], ts[T];
-    __shared__ TM pa[K * 5][T];
-    __shared__ unsigned char pj[K][T];
-    const int tid = threadIdx.x;
-    const int q = tid / 5, m = tid - 5 * q;
-    const int4 rb = rowb[blockIdx.x * kMcRows + q];
-    const int4 rl = rowl[blockIdx.x * kMcRows + q];
-    const int64_t us = uslot[blockIdx.x];
-    const TM *U = PU + us * (25 * kMcRows) + tid;
-    const int *cu = colU + us * kMcRows + q;
-    const TM *D = PD + (int64_t)blockIdx.x * (25 * kMcRows) + tid;
-    const bool act = rb.x >= 0;
-    const int i = rb.x, nin = rb.y, nup = rb.z, lev = rl.z;
-    double s = 0.0;
-    TM dg[5];
-    int col[PF];
-    pdl_trigger();
-    if (act) {
+struct McStageMany {
+    static constexpr int units = sizeof(TM) == 8 ? 200 : 400;
+};
+// Largest lists and gathered values beside it; colours that need more (rows
+// with hundreds of blocks) run unstaged.
+constexpr size_t kMcListBytes = 64u << 10;
+// Patches ahead of a CTA's own whose data it starts fetching into L2, about
+// one wave of the larger colours (96^3, FP32: 603 -> 571 us per apply).
+constexpr int kMcAheadPatches = 592;
+
+// Sum over the five lanes of a group: lane c ends with entry c of the product
+// whose part for entry (k + c) mod 5 lane c holds in p[k].
+__device__ __forceinline__ double group_sum(const double p[5], int g, int c) {
+    double v[5];
 #pragma unroll
-        for (int t = 0; t < K; t++)
-            if (t < nin) {
-                pj[t][tid] = (unsigned char)cu[t * kMcRows];
-#pragma unroll
-                for (int c = 0; c < 5; c++) pa[t * 5 + c][tid] = U[(t * 5 + c) * T];
-            }
-#pragma unroll
-        for (int c = 0; c < 5; c++) dg[c] = D[c * T];
-#pragma unroll
-        for (int t = 0; t < PF; t++) col[t] = nin + t < nup ? cu[(nin + t) * kMcRows] : 0;
-    }
-    pdl_wait();  // y and the later colours' z are complete from here on
-    if (act) {
-        s = y[(int64_t)i * 5 + m];
-#pragma unroll
-        for (int t = 0; t < PF; t++)
-            if (nin + t < nup) {
-                const double *zv = z + (int64_t)col[t] * 5;
-#pragma unroll
-                for (int c = 0; c < 5; c++) s = fma(-ld<TM>(U + ((nin + t) * 5 + c) * T), zv[c], s);
-            }
-#pragma unroll 4
-        for (int t = nin + PF; t < nup; t++) {
-            const double *zv = z + (int64_t)cu[t * kMcRows] * 5;
-#pragma unroll
-            for (int c = 0; c < 5; c++) s = fma(-ld<TM>(U + (t * 5 + c) * T), zv[c], s);
-        }
-    }
-    const int last = rl.w;
-    for (int l = 0; l <= last; l++) {
-        const bool mine = act && lev == l;
-        if (mine) {
-#pragma unroll
-            for (int t = 0; t < K; t++)
-                if (t < nin) {
-                    const double *zv = zs + pj[t][tid] * 5;
-#pragma unroll
-                    for (int c = 0; c < 5; c++) s = fma(-(double)pa[t * 5 + c][tid], zv[c], s);
-                }
-            for (int t = K; t < nin; t++) {
-                const double *zv = zs + cu[t * kMcRows] * 5;
-#pragma unroll
-                for (int c = 0; c < 5; c++) s = fma(-ld<TM>(U + (t * 5 + c) * T), zv[c], s);
-            }
-            ts[tid] = s;
-        }
-        __syncthreads();
-        if (mine) {
-            double o = 0.0;
-#pragma unroll
-            for (int c = 0; c < 5; c++) o = fma((double)dg[c], ts[q * 5 + c], o);
-            zs[tid] = o;
-        }
-        __syncthreads();
-    }
-    if (act) z[(int64_t)i * 5 + m] = zs[tid];
+    for (int k = 0; k < 5; k++) v[k] = __shfl_sync(0xffffffffu, p[k], g < 6 ? 5 * g + (c >= k ? c - k : c - k + 5) : 31);
+    return ((v[0] + v[1]) + (v[2] + v[3])) + v[4];
 }
 
-// The factors of M (factorisation order) copied into the triangular solves'
-// packed layout, one CTA per patch position: lower slot t, block entry (m, c)
-// of row q at PL[lslot * 800 + (t * 5 + c) * 160 + q * 5 + m], the upper slots
-// likewise in PU, the inverted diagonal block at PD[pos * 800 + c * 160 +
-// q * 5 + m].  Slots past a row's own count are left unwritten and never read.
-template <typename TM>
-__global__ void __launch_bounds__(5 * kMcRows) k_mc_pack(const int4 *__restrict__ rowf, const int4 *__restrict__ rowb,
-                                                        const int64_t *__restrict__ lslot,
-                                                        const int64_t *__restrict__ uslot, const TM *__restrict__ M,
-                                                        TM *__restrict__ PL, TM *__restrict__ PU,
-                                                        TM *__restrict__ PD) {
-    constexpr int T = 5 * kMcRows;
-    const int pos = blockIdx.x, tid = threadIdx.x;
-    const int q = tid / 5, m = tid - 5 * q;
-    const int4 rf = rowf[pos * kMcRows + q], rb = rowb[pos * kMcRows + q];
-    if (rf.x < 0) return;
-    const int64_t l0 = lslot[pos], u0 = uslot[pos];
-    TM *L = PL + l0 * (25 * kMcRows) + tid, *U = PU + u0 * (25 * kMcRows) + tid;
-    for (int t = 0; t < rf.z; t++) {
-        const TM *src = M + (int64_t)(rf.w + t) * 25 + m * 5;
-#pragma unroll
-        for (int c = 0; c < 5; c++) L[(t * 5 + c) * T] = src[c];
+// One triangular solve over the patches of one colour, one CTA per patch:
+// forward y = L^-1 r (OUT = y) or, BWD, backward z = U^-1 y (R = y, OUT = z).
+// Off-patch blocks couple to colours that earlier launches finished; the blocks
+// inside the patch follow its dependency levels.
+//  1. Everything constant is copied to shared memory while the previous
+//     colour still runs: the patch's lists and its region of M.
+//  2. After the dependency wait, one round trip fetches the values of the
+//     patch's distinct off-patch columns (59 on average for 140 blocks on the
+//     tet cubes) into shared memory.
+//  3. Each row subtracts its off-patch blocks.  Lane c multiplies column c, so
+//     a block costs a lane one value and five independent multiply-adds (one
+//     output per lane would load five values and chain the five
+//     multiply-adds, which bound the solve at 75-130 cycles per block).
+//  4. One warp works off the blocks inside the patch: six operations per step,
+//     on different rows and on values that earlier steps finished (scheduled
+//     at setup; about 15 steps forward, 22 backward).  The next step's blocks
+//     are already in registers, so that a step waits for one shared-memory read
+//     and five multiply-adds (some 140 cycles), never for a CTA barrier or for
+//     global memory.
+// What bounds it: latency.  A patch takes one global round trip for its
+// off-patch values and the chain of step 4, about 6,000 cycles, and three to
+// five patches share an SM.  One apply (all colours, both solves) on the tet
+// cubes, FP32 / FP64 factors: 24^3 68 / 73 us, 48^3 106 / 156 us, 96^3 521 /
+// 795 us (2.6 / 3.1 TB/s).  The row-per-five-threads form it replaces, which
+// walked the levels behind CTA barriers and read off-patch columns in chains
+// of two round trips: 173 / 202, 285 / 353 and 896 / 1178 us.
+// Slower here: one warp per patch's level walk with a row's blocks chained
+// (96^3 1130 us, FP32); all six warps walking the levels (768 us); persistent
+// CTAs with three buffers and a separate solving warp (813 us; fewer patches
+// per SM).
+template <typename TM, bool BWD, bool STAGED>
+__global__ void __launch_bounds__(kMcSolveThreads, 5) k_mc_solve(const int4 *__restrict__ desc,
+                                                              const uint4 *__restrict__ lists,
+                                                              const TM *__restrict__ M, const double *__restrict__ R,
+                                                              double *OUT, int list16, int units) {
+    extern __shared__ __align__(16) unsigned char sm[];
+    __shared__ double own[(kMcRows + 1) * 5];  // values of the patch's rows, and of idle groups
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int g = lane / 5, c = lane - 5 * g;
+    // {first 16-byte word of the lists, words, first unit of the region, units}
+    const int4 d = desc[blockIdx.x];
+    // the next colour's launch may start staging its own patches now
+    pdl_trigger();
+    const TM *G = M + (int64_t)d.z * kMcUnit;
+    const unsigned char *L = STAGED ? sm : reinterpret_cast<const unsigned char *>(lists + d.x);
+    TM *S = reinterpret_cast<TM *>(sm + (size_t)list16 * 16);
+    double *xs = reinterpret_cast<double *>(S + (size_t)units * kMcUnit);  // off-patch values
+    const int staged = STAGED ? min(d.w, units) : 0;
+    if (STAGED) {
+        uint4 *sl = reinterpret_cast<uint4 *>(sm);
+        for (int k = tid; k < d.y; k += kMcSolveThreads) copy16(sl + k, lists + d.x + k);
+        const int words = staged * (kMcUnit * (int)sizeof(TM) / 16);
+        for (int k = tid; k < words; k += kMcSolveThreads)
+            copy16(reinterpret_cast<uint4 *>(S) + k, reinterpret_cast<const uint4 *>(G) + k);
+        // a patch that a later wave of this grid takes
+        if (tid == 0 && blockIdx.x + kMcAheadPatches < gridDim.x) {
+            const int4 f = desc[blockIdx.x + kMcAheadPatches];
+            prefetch_l2(M + (int64_t)f.z * kMcUnit, (unsigned)(f.w * kMcUnit * sizeof(TM)));
+            prefetch_l2(lists + f.x, (unsigned)f.y * 16u);
+        }
+        copy_wait();
+        __syncthreads();
     }
-    for (int t = 0; t < rb.z; t++) {
-        const TM *src = M + (int64_t)(rb.w + 1 + t) * 25 + m * 5;
+    const int4 h = reinterpret_cast<const int4 *>(L)[0], h1 = reinterpret_cast<const int4 *>(L)[1];
+    const ushort2 ws = reinterpret_cast<const ushort2 *>(L + kMcWarpAt)[w];
+    const int *cols = reinterpret_cast<const int *>(L + kMcColAt);
+    const unsigned *ops = reinterpret_cast<const unsigned *>(cols + h.x);
+    const unsigned short *sidx = reinterpret_cast<const unsigned short *>(ops + 6 * h.y);
+    McGroup gr = {255, 0};
+    if (lane < 30) gr = reinterpret_cast<const McGroup *>(L + kMcGroupAt)[6 * w + g];
+    const bool act = gr.row != 255;
+    const int64_t at = ((int64_t)h.w + gr.row) * 5 + c;  // the row's entry c in R
+    if (tid < 5) own[kMcRows * 5 + tid] = 0.0;
+    double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    // r is complete before the first forward launch starts
+    if (!BWD && act) acc[0] = R[at];
+    // this thread's values of the off-patch columns: the first kGather places
+    // are read before the wait, so that their loads go out together after it
+    constexpr int kGather = 4;
+    int64_t from[kGather];
 #pragma unroll
-        for (int c = 0; c < 5; c++) U[(t * 5 + c) * T] = src[c];
+    for (int u = 0; u < kGather; u++) {
+        const int k = tid + u * kMcSolveThreads, j = k / 5;
+        from[u] = STAGED && k < 5 * h.x ? (int64_t)cols[j] * 5 + (k - 5 * j) : -1;
     }
-    const TM *dsrc = M + (int64_t)rb.w * 25 + m * 5;
+    pdl_wait();  // the earlier launches' values are complete from here on
+    if (BWD && act) acc[0] = __ldcg(R + at);
+    if (STAGED) {
+        double v[kGather];
 #pragma unroll
-    for (int c = 0; c < 5; c++) PD[(int64_t)pos * (25 * kMcRows) + c * T + tid] = dsrc[c];
+        for (int u = 0; u < kGather; u++) v[u] = from[u] >= 0 ? __ldcg(OUT + from[u]) : 0.0;
+#pragma unroll
+        for (int u = 0; u < kGather; u++)
+            if (tid + u * kMcSolveThreads < 5 * (h.x + 1)) xs[tid + u * kMcSolveThreads] = v[u];
+        for (int k = tid + kGather * kMcSolveThreads; k < 5 * (h.x + 1); k += kMcSolveThreads) {
+            const int j = k / 5;
+            xs[k] = j < h.x ? __ldcg(OUT + (int64_t)cols[j] * 5 + (k - 5 * j)) : 0.0;
+        }
+        __syncthreads();
+    }
+    const TM *in = STAGED ? S : G;  // the diagonal and intra-patch blocks are always staged
+    {
+        // slots whose elements are all staged, then the others
+        const int ns = STAGED ? max(0, staged * kMcUnit - h1.x) / kMcSlot : 0;
+        const int first = ws.x, n = ws.y;
+        const int m = min(n, max(0, ns - first));
+        int t = 0;
+        // empty places hold zeros and the index of a zero after the gathered
+        // values, so that the loops take no branch per row
+        const unsigned short *si = sidx + 6 * first + min(g, 5);
+        const int sl = min(lane, 29);
+        if (STAGED) {
+            const TM *a = S + h1.x + (size_t)first * kMcSlot + sl;
+#pragma unroll 4
+            for (; t < m; t++) {
+                const double x = xs[si[6 * t] * 5 + c];
+#pragma unroll
+                for (int k = 0; k < 5; k++) acc[k] = fma(-(double)a[t * kMcSlot + 30 * k], x, acc[k]);
+            }
+        }
+        const TM *a = G + h1.x + (size_t)first * kMcSlot + sl;
+#pragma unroll 4
+        for (; t < n; t++) {
+            const int j = si[6 * t];
+            const double x = STAGED ? xs[j * 5 + c] : j < h.x ? __ldcg(OUT + (int64_t)cols[j] * 5 + c) : 0.0;
+#pragma unroll
+            for (int k = 0; k < 5; k++) acc[k] = fma(-(double)a[t * kMcSlot + 30 * k], x, acc[k]);
+        }
+    }
+    const double s = group_sum(acc, g, c);  // entry c of the row
+    if (act) own[gr.row * 5 + c] = s;
+    __syncthreads();
+    if (w == 0) {
+        const int gg = min(g, 5);
+        const unsigned *op = ops + gg;
+        const TM *ib = in + 5 * c;
+        const int n = h.y;
+        // this step's block and the next step's operation wait in registers
+        unsigned e0 = n > 0 ? op[0] : 0u, e1 = n > 1 ? op[6] : e0;
+        TM a0[5];
+        if (n > 0) {
+#pragma unroll
+            for (int k = 0; k < 5; k++) a0[k] = ib[(e0 & 1023u) * 25 + k];
+        }
+        for (int t = 0; t < n; t++) {
+            const double *x = own + 5 * ((e0 >> 10) & 63u);
+            double *y = own + 5 * ((e0 >> 16) & 63u) + c;
+            double xv[5];
+#pragma unroll
+            for (int k = 0; k < 5; k++) xv[k] = x[k];
+            const double yv = *y;
+            TM a1[5];
+#pragma unroll
+            for (int k = 0; k < 5; k++) a1[k] = ib[(e1 & 1023u) * 25 + k];
+            const unsigned e2 = op[6 * min(t + 2, n - 1)];
+            double p = (double)a0[0] * xv[0];
+#pragma unroll
+            for (int k = 1; k < 5; k++) p = fma((double)a0[k], xv[k], p);
+            __syncwarp();
+            if (lane < 30) *y = BWD && (e0 >> 31) ? p : yv - p;
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < 5; k++) a0[k] = a1[k];
+            e0 = e1;
+            e1 = e2;
+        }
+    }
+    __syncthreads();
+    if (tid < 5 * h.z) OUT[(int64_t)h.w * 5 + tid] = own[tid];
 }
 
 }  // namespace
 
-// Ordering, slot lists, patch-local levels and the factorisation's update
-// lists (host, once per mesh).
+namespace {
+
+// The steps of a patch's solve (see mc_op): up to six operations each, on
+// different rows, an operation after those it depends on: v_row -= L v_col
+// after column col is finished; in a backward solve the diagonal operation of
+// a row after all its blocks.  Greedy, rows with the longest chain of
+// operations behind them first.
+struct McSchedule {
+    struct Op {
+        int block, row, col;  // col = row: the diagonal
+    };
+    int nr = 0;
+    bool bwd = false;
+    std::vector<Op> todo, byheight;
+    int left[kMcRows], height[kMcRows];
+    void reset(int rows, bool backward) {
+        nr = rows;
+        bwd = backward;
+        todo.clear();
+        for (int q = 0; q < nr; q++) left[q] = 0;
+    }
+    // rows in increasing order
+    void block(int b, int row, int col) {
+        todo.push_back({b, row, col});
+        left[row]++;
+    }
+    void run(std::vector<unsigned> &out) {
+        out.clear();
+        // height of a row: the longest chain of rows from its value on (at most
+        // nr).  Forward, a row's columns precede it; backward, they follow it
+        for (int q = 0; q < nr; q++) height[q] = 1;
+        const int m = (int)todo.size();
+        for (int t = 0; t < m; t++) {
+            const Op &o = todo[bwd ? t : m - 1 - t];  // rows solved last first
+            height[o.col] = std::max(height[o.col], height[o.row] + 1);
+        }
+        if (bwd)
+            for (int q = 0; q < nr; q++) todo.push_back({q, q, q});
+        // highest first, otherwise as listed
+        int at[kMcRows + 2] = {};
+        for (const Op &o : todo) at[kMcRows - height[o.row] + 1]++;
+        for (int k = 0; k <= kMcRows; k++) at[k + 1] += at[k];
+        byheight.resize(todo.size());
+        for (const Op &o : todo) byheight[at[kMcRows - height[o.row]]++] = o;
+        unsigned solved = 0;  // rows whose values are final
+        for (int q = 0; q < nr; q++)
+            if (!bwd && left[q] == 0) solved |= 1u << q;
+        while (!byheight.empty()) {
+            unsigned used = 0;
+            size_t kept = 0;
+            int k = 0;
+            Op taken[6];
+            for (size_t t = 0; t < byheight.size(); t++) {
+                const Op o = byheight[t];
+                const bool ready = o.row == o.col ? left[o.row] == 0 : (solved >> o.col) & 1u;
+                if (k < 6 && ready && !((used >> o.row) & 1u)) {
+                    used |= 1u << o.row;
+                    taken[k++] = o;
+                } else {
+                    byheight[kept++] = o;
+                }
+            }
+            byheight.resize(kept);
+            for (int g = 0; g < 6; g++) {
+                if (g >= k) {
+                    out.push_back(mc_op(0, kMcRows, kMcRows, false));
+                    continue;
+                }
+                const int q = taken[g].row;
+                const bool diag = taken[g].col == q;
+                out.push_back(mc_op(taken[g].block, taken[g].col, q, diag));
+                if (!diag) left[q]--;
+                if (bwd ? diag : left[q] == 0) solved |= 1u << q;
+            }
+        }
+    }
+};
+
+}  // namespace
+
+// Ordering, slot lists, the solves' plans and the factorisation's update lists
+// (host, once per mesh).
 int mc_build(cfd_ctx *c) {
     Abmc &mc = c->mc;
     if (mc.built) return CFD_OK;
     const int n = c->nnode;
     const std::vector<int> &IA = c->h_IA, &JA = c->h_JA, &IAU = c->h_IAU;
     const int np = (n + kMcRows - 1) / kMcRows;
+    // ranges of patches, on as many threads as their rows are worth (a row's
+    // share of a patch's loops outweighs an item of the plain ones)
+    auto parallel_patches = [&](auto fn) {
+        const int64_t items = 4 * (int64_t)n;
+        parallel_ranges(items, [&](int t, int64_t i0, int64_t i1) { fn(t, i0 * np / items, i1 * np / items); });
+    };
     // DSATUR colouring of the patch graph (Brelaz 1979): repeatedly colour the
     // uncoloured patch with the most distinct colours among its neighbours
     // (ties: most neighbours, then lowest index) with the lowest colour free
@@ -472,7 +586,7 @@ int mc_build(cfd_ctx *c) {
     // greedy colouring in patch order needs 13-14, i.e. fewer launches per
     // factorisation and per triangular solve.
     std::vector<std::vector<int>> adj(np);
-    parallel_ranges(np, [&](int, int64_t p0, int64_t p1) {
+    parallel_patches([&](int, int64_t p0, int64_t p1) {
         for (int P = (int)p0; P < (int)p1; P++) {
             const int r0 = P * kMcRows, r1 = std::min(n, r0 + kMcRows);
             for (int i = r0; i < r1; i++)
@@ -520,7 +634,6 @@ int mc_build(cfd_ctx *c) {
     auto key = [&](int j) { return (int64_t)color[j / kMcRows] * n + j; };
     std::vector<int> slot(c->nnzb), scol(c->nnzb);
     std::vector<int4> meta(n);
-    std::vector<int> lf(n, 0), lb(n, 0);
     std::vector<int> maxrow_in(range_count(n), 0);
     parallel_ranges(n, [&](int rt, int64_t i0, int64_t i1) {
     std::vector<std::pair<int64_t, int>> lo, up;
@@ -559,29 +672,156 @@ int mc_build(cfd_ctx *c) {
     parallel_ranges(c->nnzb, [&](int, int64_t u0, int64_t u1) {
         for (int64_t u = u0; u < u1; u++) scol[u] = JA[slot[u]];
     });
-    // patch-local dependency levels (a patch's rows depend only on its own rows)
-    std::vector<int2> plev(np, make_int2(0, 0));
-    parallel_ranges(np, [&](int, int64_t q0, int64_t q1) {
-    for (int P = (int)q0; P < (int)q1; P++) {
-        const int r0 = P * kMcRows, r1 = std::min(n, r0 + kMcRows);
-        for (int i = r0; i < r1; i++) {
-            int l = 0;
-            for (int u = IA[i] + meta[i].x; u < IA[i] + meta[i].y; u++) l = std::max(l, lf[scol[u]] + 1);
-            lf[i] = l;
-            plev[P].x = std::max(plev[P].x, l);
-        }
-        for (int i = r1 - 1; i >= r0; i--) {
-            int l = 0;
-            const int u0 = IA[i] + meta[i].y + 1;
-            for (int u = u0; u < u0 + meta[i].z; u++) l = std::max(l, lb[scol[u]] + 1);
-            lb[i] = l;
-            plev[P].y = std::max(plev[P].y, l);
-        }
+    // The solves' plan of each patch and direction (0 forward, 1 backward):
+    // rows to groups, the region's size, and the lists (layout at kMcWarpAt);
+    // then the regions' places in M, in launch order, and every block's place.
+    std::vector<int4> desc[2];
+    std::vector<std::vector<unsigned char>> lists[2];
+    std::vector<unsigned> loc(c->nnzb);  // first the place in the region
+    std::vector<int> ucount[2];
+    for (int dir = 0; dir < 2; dir++) {
+        desc[dir].assign(np, make_int4(0, 0, 0, 0));
+        lists[dir].resize(np);
+        ucount[dir].assign(np, 0);
     }
+    std::atomic<bool> too_long{false};
+    parallel_patches([&](int, int64_t q0, int64_t q1) {
+        std::vector<int> cols, index_of(n, -1);  // column -> its index among the patch's, -1 outside the loop below
+        int order[kMcRows];
+        std::vector<unsigned short> sidx;
+        std::vector<unsigned> ops;
+        McSchedule plan;
+        for (int pos = (int)q0; pos < (int)q1; pos++)
+            for (int dir = 0; dir < 2; dir++) {
+                const int r0 = patches[pos] * kMcRows, r1 = std::min(n, r0 + kMcRows), nr = r1 - r0;
+                // list entries of row i: intra-patch and off-patch blocks of this solve
+                auto in_at = [&](int i) { return dir ? IA[i] + meta[i].y + 1 : IA[i] + meta[i].x; };
+                auto in_n = [&](int i) { return dir ? meta[i].z : meta[i].y - meta[i].x; };
+                auto ext_at = [&](int i) { return dir ? IA[i] + meta[i].y + 1 + meta[i].z : IA[i]; };
+                auto ext_n = [&](int i) { return dir ? IA[i + 1] - ext_at(i) : meta[i].x; };
+                cols.clear();
+                int nin = 0;
+                for (int i = r0; i < r1; i++) {
+                    for (int t = 0; t < ext_n(i); t++) {
+                        const int j = scol[ext_at(i) + t];
+                        if (index_of[j] >= 0) continue;
+                        index_of[j] = 0;
+                        cols.push_back(j);
+                    }
+                    nin += in_n(i);
+                }
+                std::sort(cols.begin(), cols.end());
+                for (size_t k = 0; k < cols.size(); k++) index_of[cols[k]] = (int)k;
+                // rows by decreasing number of off-patch blocks (insertion sort)
+                for (int q = 0; q < nr; q++) {
+                    int k = q;
+                    for (; k > 0 && ext_n(r0 + order[k - 1]) < ext_n(r0 + q); k--) order[k] = order[k - 1];
+                    order[k] = q;
+                }
+                const int diag = dir ? nr : 0;
+                int slots = 0;
+                ushort2 ws[kMcWarps];
+                for (int w = 0; w < kMcWarps; w++) {
+                    const int t = 6 * w < nr ? ext_n(r0 + order[6 * w]) : 0;
+                    ws[w] = make_ushort2((unsigned short)slots, (unsigned short)t);
+                    slots += t;
+                }
+                const int64_t size = (int64_t)(diag + nin) * 25 + (int64_t)slots * kMcSlot;
+                if (slots > 65535 || cols.size() > 65534) {
+                    too_long = true;
+                    return;
+                }
+                McGroup gr[kMcGroups];
+                sidx.assign((size_t)6 * slots, (unsigned short)cols.size());
+                plan.reset(nr, dir == 1);
+                int at = 0;
+                for (int k = 0; k < kMcGroups; k++) gr[k] = {255, 0};
+                for (int k = 0; k < nr; k++) {
+                    const int q = order[k], i = r0 + q;
+                    gr[k] = {(unsigned short)q, (unsigned short)ext_n(i)};
+                    for (int t = 0; t < ext_n(i); t++) {
+                        const int u = ext_at(i) + t, at_slot = ws[k / 6].x + t;
+                        sidx[6 * at_slot + k % 6] = (unsigned short)index_of[scol[u]];
+                        loc[u] = (unsigned)(5 * (diag + nin) + (kMcSlot / 5) * at_slot + k % 6) | kMcSlotBit;
+                    }
+                }
+                for (int i = r0; i < r1; i++) {
+                    if (dir) loc[IA[i] + meta[i].y] = (unsigned)(5 * (i - r0));
+                    for (int t = 0; t < in_n(i); t++) {
+                        const int u = in_at(i) + t;
+                        loc[u] = (unsigned)(5 * (diag + at));
+                        plan.block(diag + at, i - r0, scol[u] - r0);
+                        at++;
+                    }
+                }
+                plan.run(ops);
+                for (int j : cols) index_of[j] = -1;
+                const size_t nu = cols.size(), bytes = kMcColAt + 4 * nu + 4 * ops.size() + 12 * (size_t)slots;
+                std::vector<unsigned char> &out = lists[dir][pos];
+                out.assign((bytes + 15) / 16 * 16, 0);
+                int4 *hd = reinterpret_cast<int4 *>(out.data());
+                hd[0] = make_int4((int)nu, (int)(ops.size() / 6), nr, r0);
+                hd[1] = make_int4((diag + nin) * 25, slots, 0, 0);
+                std::memcpy(out.data() + kMcWarpAt, ws, sizeof ws);
+                std::memcpy(out.data() + kMcGroupAt, gr, sizeof gr);
+                unsigned char *o = out.data() + kMcColAt;
+                auto put = [&](const void *p, size_t b) {
+                    if (b) std::memcpy(o, p, b);
+                    o += b;
+                };
+                put(cols.data(), 4 * nu);
+                put(ops.data(), 4 * ops.size());
+                put(sidx.data(), 2 * sidx.size());
+                desc[dir][pos].w = (int)((size + kMcUnit - 1) / kMcUnit);
+                ucount[dir][pos] = (int)nu;
+            }
     });
-    int maxlev = 0;
-    for (int P = 0; P < np; P++) maxlev = std::max(maxlev, std::max(plev[P].x, plev[P].y));
-    for (int i = 0; i < n; i++) meta[i].w = lf[i] | (lb[i] << 16);
+    int64_t units = 0;
+    for (int pos = 0; pos < np; pos++)
+        for (int dir = 0; dir < 2; dir++) {
+            desc[dir][pos].z = (int)units;
+            units += desc[dir][pos].w;
+        }
+    if (too_long || units * (kMcUnit / 5) >= (int64_t)kMcSlotBit) {
+        set_error("ILU(0) multicolour: too many blocks");
+        return CFD_ERR_RANGE;
+    }
+    mc.nelem = units * kMcUnit;
+    parallel_patches([&](int, int64_t q0, int64_t q1) {
+        for (int pos = (int)q0; pos < (int)q1; pos++) {
+            const int r0 = patches[pos] * kMcRows, r1 = std::min(n, r0 + kMcRows);
+            for (int i = r0; i < r1; i++)
+                for (int u = IA[i]; u < IA[i + 1]; u++)
+                    loc[u] += (unsigned)desc[u < IA[i] + meta[i].y ? 0 : 1][pos].z * (kMcUnit / 5);
+        }
+    });
+    for (int dir = 0; dir < 2; dir++) {
+        mc.shape[dir].assign(ncolor, make_int4(0, 0, 0, 0));
+        size_t words = 0;
+        for (int pos = 0; pos < np; pos++) {
+            const int w16 = (int)(lists[dir][pos].size() / 16);
+            desc[dir][pos].x = (int)words;
+            desc[dir][pos].y = w16;
+            words += w16;
+            int4 &sh = mc.shape[dir][color[patches[pos]]];
+            sh.x = std::max(sh.x, w16);
+            sh.y = std::max(sh.y, desc[dir][pos].w);
+            sh.z = std::max(sh.z, ucount[dir][pos]);
+            sh.w = std::max(sh.w, reinterpret_cast<const int4 *>(lists[dir][pos].data())[1].x);
+        }
+        if (words > (size_t)INT32_MAX) {
+            set_error("ILU(0) multicolour: patch lists too long");
+            return CFD_ERR_RANGE;
+        }
+        std::vector<unsigned char> all(words * 16);
+        parallel_patches([&](int, int64_t q0, int64_t q1) {
+            for (int pos = (int)q0; pos < (int)q1; pos++)
+                std::memcpy(all.data() + (size_t)desc[dir][pos].x * 16, lists[dir][pos].data(), lists[dir][pos].size());
+        });
+        CFD_CUDA(mc.desc[dir].upload(desc[dir].data(), desc[dir].size(), c->stream));
+        CFD_CUDA(mc.lists[dir].upload(reinterpret_cast<const uint4 *>(all.data()), words, c->stream));
+        CFD_CUDA(stream_wait(c->stream));
+    }
     // update lists of the factorisation: for lower block (i,p), the upper
     // blocks (p,j) of row p whose column j row i also holds
     // Row i's pairs in order: for each lower block u, the upper entries v of
@@ -600,11 +840,11 @@ int mc_build(cfd_ctx *c) {
                 const int j = scol[v];
                 const int *it = std::lower_bound(&JA[base], &JA[0] + end, j);
                 if (it != &JA[0] + end && *it == j) {
-                    if (out) out[total + cnt] = make_int2(v, (int)(it - &JA[base]));
+                    if (out) out[total + cnt] = make_int2((int)loc[v], (int)(it - &JA[base]));
                     cnt++;
                 }
             }
-            if (out) hdr[base + u] = make_int4(IA[p] + meta[p].y, cnt, kk - base, 0);
+            if (out) hdr[base + u] = make_int4((int)loc[IA[p] + meta[p].y], cnt, kk - base, 0);
             total += cnt;
         }
         return total;
@@ -621,66 +861,12 @@ int mc_build(cfd_ctx *c) {
     parallel_ranges(n, [&](int, int64_t i0, int64_t i1) {
         for (int i = (int)i0; i < (int)i1; i++) row_pairs(i, pairs.data() + pair_ptr[i]);
     });
-    // row records and packed-layout slots of the triangular solves, in launch
-    // order (colour, then position of the patch in the colour, then row)
-    std::vector<int4> rowf((size_t)np * kMcRows), rowb((size_t)np * kMcRows), rowl((size_t)np * kMcRows);
-    std::vector<int64_t> lslot(np + 1, 0), uslot(np + 1, 0);
-    for (int pos = 0; pos < np; pos++) {
-        const int P = patches[pos];
-        int lmax = 0, umax = 0;
-        for (int q = 0; q < kMcRows; q++) {
-            const int i = P * kMcRows + q;
-            const size_t e = (size_t)pos * kMcRows + q;
-            if (i < n) {
-                const int base = IA[i], diag = base + meta[i].y;
-                rowf[e] = make_int4(i, meta[i].x, meta[i].y, base);
-                rowb[e] = make_int4(i, meta[i].z, IA[i + 1] - diag - 1, diag);
-                rowl[e] = make_int4(lf[i], plev[P].x, lb[i], plev[P].y);
-                lmax = std::max(lmax, meta[i].y);
-                umax = std::max(umax, IA[i + 1] - diag - 1);
-            } else {
-                rowf[e] = rowb[e] = make_int4(-1, 0, 0, 0);
-                rowl[e] = make_int4(-1, plev[P].x, -1, plev[P].y);
-            }
-        }
-        lslot[pos + 1] = lslot[pos] + lmax;
-        uslot[pos + 1] = uslot[pos] + umax;
-    }
-    std::vector<int> colL((size_t)lslot[np] * kMcRows, 0), colU((size_t)uslot[np] * kMcRows, 0);
-    parallel_ranges(np, [&](int, int64_t q0, int64_t q1) {
-    for (int pos = (int)q0; pos < (int)q1; pos++) {
-        const int p0 = patches[pos] * kMcRows;
-        for (int q = 0; q < kMcRows; q++) {
-            const int4 rf = rowf[(size_t)pos * kMcRows + q], rb = rowb[(size_t)pos * kMcRows + q];
-            if (rf.x < 0) continue;
-            for (int t = 0; t < rf.z; t++) {
-                const int j = scol[rf.w + t];
-                colL[(size_t)(lslot[pos] + t) * kMcRows + q] = t < rf.y ? j : j - p0;
-            }
-            for (int t = 0; t < rb.z; t++) {
-                const int j = scol[rb.w + 1 + t];
-                colU[(size_t)(uslot[pos] + t) * kMcRows + q] = t < rb.y ? j - p0 : j;
-            }
-        }
-    }
-    });
-    mc.nlslot = lslot[np];
-    mc.nuslot = uslot[np];
-    CFD_CUDA(mc.rowf.upload(rowf.data(), rowf.size(), c->stream));
-    CFD_CUDA(mc.rowb.upload(rowb.data(), rowb.size(), c->stream));
-    CFD_CUDA(mc.rowl.upload(rowl.data(), rowl.size(), c->stream));
-    CFD_CUDA(mc.lslot.upload(lslot.data(), lslot.size(), c->stream));
-    CFD_CUDA(mc.uslot.upload(uslot.data(), uslot.size(), c->stream));
-    CFD_CUDA(mc.colL.upload(colL.data(), std::max<size_t>(1, colL.size()), c->stream));
-    CFD_CUDA(mc.colU.upload(colU.data(), std::max<size_t>(1, colU.size()), c->stream));
     mc.maxrow = maxrow;
-    mc.maxlev = maxlev;
     mc.maxstage = maxstage;
     CFD_CUDA(mc.patches.upload(patches.data(), patches.size(), c->stream));
     CFD_CUDA(mc.slot.upload(slot.data(), slot.size(), c->stream));
-    CFD_CUDA(mc.scol.upload(scol.data(), scol.size(), c->stream));
     CFD_CUDA(mc.meta.upload(meta.data(), meta.size(), c->stream));
-    CFD_CUDA(mc.plev.upload(plev.data(), plev.size(), c->stream));
+    CFD_CUDA(mc.loc.upload(loc.data(), loc.size(), c->stream));
     CFD_CUDA(mc.hdr.upload(hdr.data(), hdr.size(), c->stream));
     CFD_CUDA(mc.pair_ptr.upload(pair_ptr.data(), pair_ptr.size(), c->stream));
     CFD_CUDA(mc.pairs.upload(pairs.data(), (size_t)pair_ptr[n], c->stream));
@@ -706,68 +892,63 @@ int mc_factor(cfd_ctx *c, const TA *A, TM *M) {
     const size_t smem = per_warp * nwarp;
     int smax = 0;
     CFD_CUDA(allow_max_dynamic_smem(k_mc_factor<TA, TM>, c->device, &smax));
+    CFD_CUDA(allow_max_dynamic_smem(k_mc_solve<TM, false, true>, c->device, nullptr));
+    CFD_CUDA(allow_max_dynamic_smem(k_mc_solve<TM, true, true>, c->device, nullptr));
     if (smem > (size_t)smax) {
         set_error("ILU(0) multicolour: %zu bytes of shared memory needed, %d available", smem, smax);
         return CFD_ERR_RANGE;
     }
+    // the slots' empty places read as zeros
+    CFD_CUDA(cudaMemsetAsync(M, 0, (size_t)mc.nelem * sizeof(TM), c->stream));
     for (int k = 0; k < mc.ncolor; k++) {
         const int cnt = mc.cptr[k + 1] - mc.cptr[k];
         k_mc_factor<TA, TM><<<grid_for(cnt, nwarp), 32 * nwarp, smem, c->stream>>>(
             mc.patches.p + mc.cptr[k], cnt, c->nnode, mc.maxrow, mc.maxstage, c->IA.p, mc.slot.p, mc.meta.p,
-            mc.hdr.p, mc.pair_ptr.p, mc.pairs.p, A, M, c->err.p);
+            mc.hdr.p, mc.loc.p, mc.pair_ptr.p, mc.pairs.p, A, M, c->err.p);
     }
     CFD_LAUNCH_CHECK();
-    // the triangular solves read the factors in their packed layout
-    McPack<TM> &pk = mc.pack<TM>();
-    const int np = mc.cptr[mc.ncolor];
-    const size_t nl = (size_t)mc.nlslot * 25 * kMcRows, nu = (size_t)mc.nuslot * 25 * kMcRows,
-                 nd = (size_t)np * 25 * kMcRows;
-    if (pk.L.n != std::max<size_t>(1, nl) || pk.U.n != std::max<size_t>(1, nu) || pk.D.n != nd) {
-        mc.clear_graphs();  // captured applies hold the old addresses
-        CFD_CUDA(pk.L.alloc(std::max<size_t>(1, nl)));
-        CFD_CUDA(pk.U.alloc(std::max<size_t>(1, nu)));
-        CFD_CUDA(pk.D.alloc(nd));
-    }
-    k_mc_pack<TM><<<np, 5 * kMcRows, 0, c->stream>>>(mc.rowf.p, mc.rowb.p, mc.lslot.p, mc.uslot.p, M, pk.L.p, pk.U.p,
-                                                      pk.D.p);
-    CFD_LAUNCH_CHECK();
+    return CFD_OK;
+}
+
+template <typename TM, bool BWD>
+static int mc_solve_launch(cfd_ctx *c, int k, bool dependent, const TM *M, const double *r, double *out) {
+    const Abmc &mc = c->mc;
+    const int4 sh = mc.shape[BWD][k];
+    const int npatch = mc.cptr[k + 1] - mc.cptr[k];
+    const size_t lists = (size_t)sh.x * 16 + ((size_t)sh.z + 1) * 40;
+    // the diagonal and intra-patch blocks are staged whole or not at all
+    const bool staged = lists <= kMcListBytes && sh.w <= kMcStageUnits * kMcUnit;
+    auto bytes = [&](int units) { return lists + (size_t)units * kMcUnit * sizeof(TM); };
+    int units = std::min(sh.y, kMcStageUnits);
+    if ((size_t)npatch > (size_t)c->nsm * ((220u << 10) / (bytes(units) + 3072)))
+        units = std::min(units, std::max(McStageMany<TM>::units, (sh.w + kMcUnit - 1) / kMcUnit));
+    if (!staged) units = 0;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3(npatch);
+    lc.blockDim = dim3(kMcSolveThreads);
+    lc.dynamicSmemBytes = staged ? bytes(units) : 0;
+    lc.stream = c->stream;
+    lc.attrs = at;
+    lc.numAttrs = dependent ? 1 : 0;
+    auto kern = staged ? k_mc_solve<TM, BWD, true> : k_mc_solve<TM, BWD, false>;
+    CFD_CUDA(cudaLaunchKernelEx(&lc, kern, (const int4 *)(mc.desc[BWD].p + mc.cptr[k]), (const uint4 *)mc.lists[BWD].p,
+                                M, r, out, sh.x, units));
     return CFD_OK;
 }
 
 template <typename TM>
 static int mc_apply_launch(cfd_ctx *c, const TM *M, const double *r, double *tmp, double *z) {
-    Abmc &mc = c->mc;
-    (void)M;  // the solves read the packed copy mc_factor made of M
-    struct {
-        const TM *L, *U, *D;
-    } pk{mc.pack<TM>().L.p, mc.pack<TM>().U.p, mc.pack<TM>().D.p};
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t lc = {};
-    lc.blockDim = dim3(5 * kMcRows);
-    lc.dynamicSmemBytes = 0;
-    lc.stream = c->stream;
-    lc.attrs = at;
-    lc.numAttrs = 1;
-    for (int k = 0; k < mc.ncolor; k++) {
-        lc.gridDim = dim3(mc.cptr[k + 1] - mc.cptr[k]);
-        // the first colour starts after the stream's earlier work has completed
-        // (no early start), so r is complete in every colour's launch
-        lc.numAttrs = k == 0 ? 0 : 1;
-        const size_t e = (size_t)mc.cptr[k] * kMcRows;
-        CFD_CUDA(cudaLaunchKernelEx(&lc, k_mc_fwd<TM>, (const int4 *)(mc.rowf.p + e), (const int4 *)(mc.rowl.p + e),
-                                    (const int64_t *)(mc.lslot.p + mc.cptr[k]), (const int *)mc.colL.p,
-                                    (const TM *)pk.L, r, tmp));
-    }
-    lc.numAttrs = 1;
-    for (int k = mc.ncolor - 1; k >= 0; k--) {
-        lc.gridDim = dim3(mc.cptr[k + 1] - mc.cptr[k]);
-        const size_t e = (size_t)mc.cptr[k] * kMcRows;
-        CFD_CUDA(cudaLaunchKernelEx(&lc, k_mc_bwd<TM>, (const int4 *)(mc.rowb.p + e), (const int4 *)(mc.rowl.p + e),
-                                    (const int64_t *)(mc.uslot.p + mc.cptr[k]), (const int *)mc.colU.p,
-                                    (const TM *)pk.U, (const TM *)(pk.D + e * 25), (const double *)tmp, z));
-    }
+    const Abmc &mc = c->mc;
+    int st;
+    // the first colour starts after the stream's earlier work has completed
+    // (no early start), so r is complete in every colour's launch
+    for (int k = 0; k < mc.ncolor; k++)
+        if ((st = mc_solve_launch<TM, false>(c, k, k > 0, M, r, tmp))) return st;
+    for (int k = mc.ncolor - 1; k >= 0; k--)
+        if ((st = mc_solve_launch<TM, true>(c, k, true, M, tmp, z))) return st;
     CFD_LAUNCH_CHECK();
     return CFD_OK;
 }

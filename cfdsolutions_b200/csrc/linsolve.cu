@@ -675,13 +675,13 @@ static int precond_setup(cfd_ctx *c, const Precond &pc) {
     if (pc.kind == CFD_PC_ILU0_MC) {
         // block multicolour order: factors read straight from the stored
         // matrix (its own precision), FP64 arithmetic, stored in pc.prec
+        int st = mc_build(c);
+        if (st) return st;
         if (pc.prec == CFD_PREC_FP64) {
-            CFD_CUDA(c->M64.alloc(nz));
-            int st = mc_factor<double, double>(c, c->A64.p, c->M64.p);
-            if (st) return st;
+            CFD_CUDA(c->M64.alloc((size_t)c->mc.nelem));
+            if ((st = mc_factor<double, double>(c, c->A64.p, c->M64.p))) return st;
         } else {
-            CFD_CUDA(c->M32.alloc(nz));
-            int st;
+            CFD_CUDA(c->M32.alloc((size_t)c->mc.nelem));
             if (c->a_precision == CFD_PREC_FP32 && c->A32.p) st = mc_factor<float, float>(c, c->A32.p, c->M32.p);
             else if (c->a_precision == CFD_PREC_BF16 && c->A16.p)
                 st = mc_factor<uint16_t, float>(c, c->A16.p, c->M32.p);

@@ -51,8 +51,8 @@ double unit_pm1(uint64_t seed, uint64_t k) {
 // Device bytes of one request, from the box dimensions (the mesh is built
 // after admission): per node the state, residuals, gradients, limiters (two
 // buffers), geometry, incidence and (restart+1)+5 Krylov/work vectors; per block of the
-// Jacobian its stored copies, the preconditioner factors (three times their
-// size: the factors and the triangular solves' padded packed copy) and the
+// Jacobian its stored copies, the preconditioner factors (counted three times;
+// they take 1.1 times their size, with the empty places of their slots) and the
 // ordering lists.  A tet-split box has ~7 interior edges per node, blocks = N + 2E.
 double estimate_bytes(const cfd_serve_request &r) {
     const double N = (double)(r.nx + 1) * (r.ny + 1) * (r.nz + 1);
