@@ -11,6 +11,7 @@
 #include <cstdio>
 #include <cstring>
 #include <numeric>
+#include <type_traits>
 #include <vector>
 
 #include "ctx.cuh"
@@ -627,180 +628,71 @@ __global__ void k_add_diss(int64_t n, const double *__restrict__ a, const double
 // ---- approximate Roe Jacobian (Compute_Jacobian_Approximate_Roe,
 //      Euler3D/src/Roe_Jacobian.cpp:29-228)
 
-// Off-diagonal blocks, one thread per interior edge:
-//   A[L,R] = dFdR = 0.5 (J(Q_R) - |A|) area,  A[R,L] = -dFdL = -0.5 (J(Q_L) + |A|) area.
-// Every off-diagonal slot belongs to exactly one edge, so no zeroing and no
-// accumulation is needed.
-// MODE: 0 Roe, 1 preconditioned Roe (CFD_FLUX_ROE_PRECOND), 2 Thornber (|A| of the modified states)
-constexpr int JAC_WARPS = 4;  // warps per CTA of k_jac_edges / k_jac_rows_warp
-
-template <typename TA, int MODE>
-__global__ void __launch_bounds__(128) k_jac_edges(int nedge, int64_t ldq, const double *__restrict__ Q,
-                                                   const int2 *__restrict__ en, const double4 *__restrict__ eg,
-                                                   const int2 *__restrict__ eslot, Flow f, double *__restrict__ A64,
-                                                   TA *__restrict__ Alow) {
-    // Each block is stored by the warp together: the lanes put their blocks in
-    // shared memory and the warp then writes them one after the other, lane m
-    // element m, so every block leaves as one contiguous 100/200-byte store
-    // instead of 25 scalar stores scattered over 32 slots.
-    __shared__ double stage[JAC_WARPS][32][26];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e - lane >= nedge) return;  // whole warps past the end
-    const bool live = e < nedge;
-    const int2 nd = en[live ? e : nedge - 1];
-    const double4 g = eg[live ? e : nedge - 1];
-    double qL[5], qR[5];
-#pragma unroll
-    for (int v = 0; v < 5; v++) {
-        qL[v] = Q[v * ldq + nd.x];
-        qR[v] = Q[v * ldq + nd.y];
-    }
-    double Ab[25], J[25];
-    if (MODE == 1) {
-        pc_abs_jacobian(qL, qR, g.x, g.y, g.z, f, Ab);
-    } else if (MODE == 2) {
-        double mL[5], mR[5];
-        thornber_states(qL, qR, f, mL, mR);
-        roe_abs_jacobian(mL, mR, g.x, g.y, g.z, f, Ab);
-    } else {
-        roe_abs_jacobian(qL, qR, g.x, g.y, g.z, f, Ab);
-    }
-    const int2 sl = eslot[live ? e : nedge - 1];
-    const double ha = 0.5 * g.w;
-    const unsigned act = __ballot_sync(0xffffffffu, live);
-    for (int half = 0; half < 2; half++) {
-        flux_jacobian(half == 0 ? qR : qL, g.x, g.y, g.z, f, J);
-#pragma unroll
-        for (int k = 0; k < 25; k++) stage[w][lane][k] = half == 0 ? ha * (J[k] - Ab[k]) : -ha * (J[k] + Ab[k]);
-        __syncwarp();
-        const int myslot = half == 0 ? sl.x : sl.y;
-        for (int b = 0; b < 32; b++) {
-            const int slot = __shfl_sync(0xffffffffu, myslot, b);
-            if (!((act >> b) & 1u) || lane >= 25) continue;
-            const double val = stage[w][b][lane];
-            if (A64) A64[(int64_t)slot * 25 + lane] = val;
-            if (Alow) store_low(Alow + (int64_t)slot * 25 + lane, val);
-        }
-        __syncwarp();
-    }
-}
-
-// Diagonal blocks and right-hand side, one thread per row:
+// Blocks of an interior edge (L,R): A[L,R] = 0.5 (J(Q_R) - |A|) area,
+// A[R,L] = -0.5 (J(Q_L) + |A|) area; the rows' diagonal blocks and right-hand
+// sides:
 //   A[i,i] = V_i/dt_i I - sum_j A[j,i] + sum_b 0.5 (J(Q_i) + |A|)_b area_b
 //   B_i    = -(Res_i [+ Res_Diss_i])
-// One warp per row without boundary edges (the rows with boundary edges go to
-// k_jac_rows, one thread per row): lane m < 25 owns element m of the diagonal
-// block, so each transposed off-diagonal block is one contiguous read of the
-// warp; lanes 0-4 form B.  Same terms in the same order as k_jac_rows.
-template <typename TA, int MODE>
-__global__ void __launch_bounds__(32 * JAC_WARPS) k_jac_rows_warp(
-    int nnode, int64_t ldq, const double *__restrict__ Q, const int *__restrict__ IA, const int *__restrict__ IAU,
-    const int *__restrict__ tslot, const int *__restrict__ n2b_ptr, const double *__restrict__ vol,
-    const double *__restrict__ dt, const double *__restrict__ res, const double *__restrict__ resd, int add_time,
-    int include_diss, Flow f, double *__restrict__ A64, TA *__restrict__ Alow, double *__restrict__ B) {
-    const int lane = threadIdx.x & 31;
-    const int i = blockIdx.x * JAC_WARPS + (threadIdx.x >> 5);
-    if (i >= nnode || n2b_ptr[i + 1] > n2b_ptr[i]) return;  // whole warps
-    const int m = lane < 25 ? lane : 24;
-    const double vd = add_time ? vol[i] / dt[i] : 0.0;
-    double d;
-    if (MODE == 1 && add_time) {
-        double qi[5], C[25];
-#pragma unroll
-        for (int v = 0; v < 5; v++) qi[v] = Q[v * ldq + i];
-        pc_node_cinv(qi, f, C);
-        double cm = C[0];
-#pragma unroll
-        for (int k = 1; k < 25; k++)
-            if (k == m) cm = C[k];
-        d = cm * vd;
-    } else if (f.rup && add_time) {
-        // (V/dt) dQ/d(rho,u,v,w,p) (Roe_Jacobian.cpp:241-264 with PRECOND_METHOD_NONE)
-        double qi[5], M[25];
-#pragma unroll
-        for (int v = 0; v < 5; v++) qi[v] = Q[v * ldq + i];
-        state_time_matrix(qi, f, M);
-        double cm = M[0];
-#pragma unroll
-        for (int k = 1; k < 25; k++)
-            if (k == m) cm = M[k];
-        d = cm * vd;
-    } else {
-        d = (m % 6 == 0) ? vd : 0.0;
-    }
-    const int dg = IAU[i];
-    for (int k = IA[i]; k < IA[i + 1]; k++) {
-        if (k == dg) continue;
-        const int64_t b = (int64_t)tslot[k] * 25 + m;
-        d -= A64 ? A64[b] : load_low(Alow + b);
-    }
-    if (lane < 25) {
-        if (A64) A64[(int64_t)dg * 25 + lane] = d;
-        if (Alow) store_low(Alow + (int64_t)dg * 25 + lane, d);
-    }
-    if (lane < 5) {
-        double r = res[lane * (int64_t)nnode + i];
-        if (include_diss) r += resd[lane * (int64_t)nnode + i];
-        B[(int64_t)i * 5 + lane] = -r;
-    }
+// One thread per row walks its edges (the sliced-ELL incidence, whose order is
+// that of the row's blocks) and forms both blocks of each: its own, stored,
+// and the transposed one, added to its diagonal block in registers.  Every edge
+// is evaluated from both ends, in the same orientation and so to the same bits,
+// and no block is read back: the two passes this replaces (edges, then rows
+// that gathered the transposed blocks) moved the blocks three times, half of
+// it in partial sectors.  Measured on the 96^3 cube, FP32 / FP64 blocks: 1067 /
+// 1268 us (before: 1430 / 1632), 24^3 43 / 41 us (58 / 61).  Bound by the FP64
+// pipe and by latency at three CTAs per SM (168 registers).  The lanes stage their blocks in
+// shared memory and the warp stores them one after the other, 100 or 200
+// contiguous bytes each; a row's next block follows in the next step, so the
+// sectors they share fill in L2.
+// The low-precision-only system sums the diagonal from the rounded blocks.
+// MODE: 0 Roe, 1 preconditioned Roe (CFD_FLUX_ROE_PRECOND), 2 Thornber (|A| of
+// the modified states).  RUP: the state's variables (f.rup).  HIGH / LOW: an
+// FP64 / a low-precision matrix is stored.
+constexpr int JAC_WARPS = 4;  // warps per CTA
+
+template <typename TA>
+__device__ __forceinline__ double round_low(double v) {
+    TA t;
+    store_low(&t, v);
+    return load_low(&t);
 }
 
-template <typename TA, int MODE>
-__global__ void __launch_bounds__(128) k_jac_rows(
-    int nrows, const int *__restrict__ rows, int64_t ldq, const double *__restrict__ Q, const int *__restrict__ IA,
-    const int *__restrict__ IAU, const int *__restrict__ tslot, const int *__restrict__ n2b_ptr,
-    const int *__restrict__ n2b, const int2 *__restrict__ bn, const double4 *__restrict__ bg,
-    const double *__restrict__ vol, const double *__restrict__ dt, const double *__restrict__ res,
-    const double *__restrict__ resd, int add_time, int include_diss, Flow f, int nnode, double *__restrict__ A64,
-    TA *__restrict__ Alow, double *__restrict__ B) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nrows) return;
-    const int i = rows[t];
-    double D[25];
-    const double vd = add_time ? vol[i] / dt[i] : 0.0;
+template <typename TA, int MODE, bool RUP, bool HIGH, bool LOW>
+__global__ void __launch_bounds__(32 * JAC_WARPS, MODE == 1 ? 2 : 3) k_jacobian(
+    int nnode, int64_t ldq, const double *__restrict__ Q, const int *__restrict__ IA, const int *__restrict__ IAU,
+    const int64_t *__restrict__ sell_ptr, const int *__restrict__ sell_nbr, const double4 *__restrict__ sell_geo,
+    const int *__restrict__ deg, const int *__restrict__ n2b_ptr, const int *__restrict__ n2b,
+    const int2 *__restrict__ bn, const double4 *__restrict__ bg, const double *__restrict__ vol,
+    const double *__restrict__ dt, const double *__restrict__ res, const double *__restrict__ resd, int add_time,
+    int include_diss, Flow f, double *__restrict__ A64, TA *__restrict__ Alow, double *__restrict__ B) {
+    f.rup = RUP ? 1 : 0;  // a compile-time constant below
+    using TS = std::conditional_t<HIGH, double, TA>;  // staged blocks
+    __shared__ TS stage[JAC_WARPS][32][25];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i - lane >= nnode) return;  // whole warps past the end
+    const bool live = i < nnode;
+    const int row = live ? i : nnode - 1;
+    const int d = live ? deg[row] : 0, first = IA[row], end = IA[row + 1];
+    const int64_t base = sell_ptr[row >> 5] + lane;
+    const int steps = (int)((sell_ptr[(row >> 5) + 1] - sell_ptr[row >> 5]) / 32);
+    double qi[5], D[25];
+#pragma unroll
+    for (int v = 0; v < 5; v++) qi[v] = Q[v * ldq + row];
+    const double vd = add_time ? vol[row] / dt[row] : 0.0;
     if (MODE == 1 && add_time) {
         // preconditioned pseudo-time term (V/dt) Cinv (Roe_Jacobian.cpp:241-264)
-        double qi[5];
-#pragma unroll
-        for (int v = 0; v < 5; v++) qi[v] = Q[v * ldq + i];
         pc_node_cinv(qi, f, D);
 #pragma unroll
         for (int k = 0; k < 25; k++) D[k] *= vd;
-    } else if (f.rup && add_time) {
-        double qi[5];
-#pragma unroll
-        for (int v = 0; v < 5; v++) qi[v] = Q[v * ldq + i];
+    } else {
+        // (V/dt) dQ/dW
         state_time_matrix(qi, f, D);
 #pragma unroll
         for (int k = 0; k < 25; k++) D[k] *= vd;
-    } else {
-#pragma unroll
-        for (int k = 0; k < 25; k++) D[k] = (k % 6 == 0) ? vd : 0.0;
     }
-    const int dg = IAU[i];
-    for (int k = IA[i]; k < IA[i + 1]; k++) {
-        if (k == dg) continue;
-        if (A64) {
-            const double *blk = A64 + (int64_t)tslot[k] * 25;
-#pragma unroll
-            for (int m = 0; m < 25; m++) D[m] -= blk[m];
-        } else {  // low-precision-only system: sum the stored blocks
-            const TA *blk = Alow + (int64_t)tslot[k] * 25;
-#pragma unroll
-            for (int m = 0; m < 25; m++) D[m] -= load_low(blk + m);
-        }
-    }
-    for (int k = n2b_ptr[i]; k < n2b_ptr[i + 1]; k++) {
-        const int b = n2b[k];
-        const int2 nd = bn[b];
-        const double4 g = bg[b];
-        double qL[5], qR[5], Ab[25], J[25];
-#pragma unroll
-        for (int v = 0; v < 5; v++) {
-            qL[v] = Q[v * ldq + nd.x];
-            qR[v] = Q[v * ldq + nd.y];
-        }
+    auto dissipation = [&](const double qL[5], const double qR[5], const double4 &g, double Ab[25]) {
         if (MODE == 1) {
             pc_abs_jacobian(qL, qR, g.x, g.y, g.z, f, Ab);
         } else if (MODE == 2) {
@@ -810,40 +702,99 @@ __global__ void __launch_bounds__(128) k_jac_rows(
         } else {
             roe_abs_jacobian(qL, qR, g.x, g.y, g.z, f, Ab);
         }
-        flux_jacobian(qL, g.x, g.y, g.z, f, J);
-        const double ha = 0.5 * g.w;
+    };
+    // the warp's staged blocks to their slots, lane m element m; slot < 0: none
+    auto store = [&](int slot) {
+        __syncwarp();
+        for (int b = 0; b < 32; b++) {
+            const int at = __shfl_sync(0xffffffffu, slot, b);
+            if (at < 0 || lane >= 25) continue;
+            const TS v = stage[w][b][lane];
+            if (HIGH) A64[(int64_t)at * 25 + lane] = v;
+            if (LOW) {
+                if constexpr (HIGH) store_low(Alow + (int64_t)at * 25 + lane, v);
+                else Alow[(int64_t)at * 25 + lane] = v;
+            }
+        }
+        __syncwarp();
+    };
+    auto put = [&](int k, double v) {
+        if constexpr (HIGH) stage[w][lane][k] = v;
+        else store_low(&stage[w][lane][k], v);
+    };
+    for (int k = 0; k < steps; k++) {
+        int slot = -1;
+        if (k < d) {
+            const int sn = sell_nbr[base + 32 * k];
+            const double4 g = sell_geo[base + 32 * k];
+            const bool own_is_L = sn >= 0;
+            const int j = own_is_L ? sn : ~sn;
+            double qj[5], qL[5], qR[5];
 #pragma unroll
-        for (int m = 0; m < 25; m++) D[m] += ha * (J[m] + Ab[m]);
+            for (int v = 0; v < 5; v++) {
+                qj[v] = Q[v * ldq + j];
+                qL[v] = own_is_L ? qi[v] : qj[v];
+                qR[v] = own_is_L ? qj[v] : qi[v];
+            }
+            double Ab[25], J[25];
+            dissipation(qL, qR, g, Ab);
+            // own block 0.5 (+-J(Q_j) - |A|) area, transposed one 0.5 (-+J(Q_i) - |A|) area
+            const double ha = 0.5 * g.w, sg = own_is_L ? 1.0 : -1.0;
+            flux_jacobian(qj, g.x, g.y, g.z, f, J);
+#pragma unroll
+            for (int m = 0; m < 25; m++) put(m, ha * (sg * J[m] - Ab[m]));
+            flux_jacobian(qi, g.x, g.y, g.z, f, J);
+#pragma unroll
+            for (int m = 0; m < 25; m++) {
+                const double other = ha * (-sg * J[m] - Ab[m]);
+                D[m] -= HIGH ? other : round_low<TA>(other);
+            }
+            // block k of the row, the diagonal one lying before those of larger columns
+            slot = first + k + (j > row ? 1 : 0);
+            if (slot >= end) slot = -1;
+        }
+        store(slot);
     }
+    if (live)
+        for (int k = n2b_ptr[row]; k < n2b_ptr[row + 1]; k++) {
+            const int b = n2b[k];
+            const int2 nd = bn[b];
+            const double4 g = bg[b];
+            double qR[5], Ab[25], J[25];
 #pragma unroll
-    for (int m = 0; m < 25; m++) {
-        if (A64) A64[(int64_t)dg * 25 + m] = D[m];
-        if (Alow) store_low(Alow + (int64_t)dg * 25 + m, D[m]);
-    }
+            for (int v = 0; v < 5; v++) qR[v] = Q[v * ldq + nd.y];
+            dissipation(qi, qR, g, Ab);
+            flux_jacobian(qi, g.x, g.y, g.z, f, J);
+            const double ha = 0.5 * g.w;
 #pragma unroll
-    for (int v = 0; v < 5; v++) {
-        double r = res[v * (int64_t)nnode + i];
-        if (include_diss) r += resd[v * (int64_t)nnode + i];
-        B[(int64_t)i * 5 + v] = -r;
+            for (int m = 0; m < 25; m++) D[m] += ha * (J[m] + Ab[m]);
+        }
+#pragma unroll
+    for (int m = 0; m < 25; m++) put(m, D[m]);
+    store(live ? IAU[row] : -1);
+    if (live) {
+#pragma unroll
+        for (int v = 0; v < 5; v++) {
+            double r = res[v * (int64_t)nnode + row];
+            if (include_diss) r += resd[v * (int64_t)nnode + row];
+            B[(int64_t)row * 5 + v] = -r;
+        }
     }
 }
 
-// Edge blocks then diagonal blocks and right-hand side of the approximate
-// Roe Jacobian (MODE as k_jac_edges).
+// The approximate Roe Jacobian and right-hand side (MODE as k_jacobian).
 template <typename TA, int MODE>
 static void launch_jacobian(cfd_ctx *c, int add_time, int include_diss, double *A64, TA *Alow) {
-    const int ge = grid_for(c->nedge, 32 * JAC_WARPS);
-    if (c->nedge)
-        k_jac_edges<TA, MODE><<<ge, 32 * JAC_WARPS, 0, c->stream>>>(c->nedge, c->ldq, c->Q.p, c->edge_nodes.p,
-                                                                  c->edge_geo.p, c->eslot.p, c->flow, A64, Alow);
-    k_jac_rows_warp<TA, MODE><<<grid_for(c->nnode, JAC_WARPS), 32 * JAC_WARPS, 0, c->stream>>>(
-        c->nnode, c->ldq, c->Q.p, c->IA.p, c->IAU.p, c->tslot.p, c->n2b_ptr.p, c->cvol.p, c->dt.p, c->res.p,
-        c->resd.p, add_time, include_diss, c->flow, A64, Alow, c->B.p);
-    if (c->nbnode > 0)
-        k_jac_rows<TA, MODE><<<grid_for(c->nbnode, 128), 128, 0, c->stream>>>(
-            c->nbnode, c->bnode.p, c->ldq, c->Q.p, c->IA.p, c->IAU.p, c->tslot.p, c->n2b_ptr.p, c->n2b.p,
-            c->bedge_nodes.p, c->bedge_geo.p, c->cvol.p, c->dt.p, c->res.p, c->resd.p, add_time, include_diss,
-            c->flow, c->nnode, A64, Alow, c->B.p);
+    auto run = [&](auto kern) {
+        kern<<<grid_for(c->nnode, 32 * JAC_WARPS), 32 * JAC_WARPS, 0, c->stream>>>(
+            c->nnode, c->ldq, c->Q.p, c->IA.p, c->IAU.p, c->sell_ptr.p, c->sell_nbr.p, c->sell_geo.p, c->deg.p,
+            c->n2b_ptr.p, c->n2b.p, c->bedge_nodes.p, c->bedge_geo.p, c->cvol.p, c->dt.p, c->res.p, c->resd.p,
+            add_time, include_diss, c->flow, A64, Alow, c->B.p);
+    };
+    const bool rup = c->flow.rup != 0;
+    if (A64 && Alow) run(rup ? k_jacobian<TA, MODE, true, true, true> : k_jacobian<TA, MODE, false, true, true>);
+    else if (A64) run(rup ? k_jacobian<TA, MODE, true, true, false> : k_jacobian<TA, MODE, false, true, false>);
+    else run(rup ? k_jacobian<TA, MODE, true, false, true> : k_jacobian<TA, MODE, false, false, true>);
 }
 
 template <typename TA>

@@ -360,9 +360,14 @@ __device__ __forceinline__ void state_time_matrix(const double q[5], const Flow 
 }
 
 // Roe dissipation matrix |A| = M P |Lambda| P^-1 M^-1 (Compute_RoeAJacobian,
-// Euler3D/src/Roe_Fluxes.cpp:149-273), assembled as M * D * M^-1 where
-// D = P |Lambda| P^-1 is written out in closed form in the (rho,u,v,w,p)
-// variables -- the same matrix whose action on dq is the flux's dw.
+// Euler3D/src/Roe_Fluxes.cpp:149-273) at the Roe average, as the multiple of
+// the identity and the two rank-one terms it consists of: with dp and dU the
+// jumps of the pressure and the normal velocity that dQ stands for,
+//   |A| dQ = E0 dQ + (Es/2 dp / c^2 + Ed/2 rho dU / c) (1,u,v,w,H) + (Es/2 rho dU + Ed/2 dp / c) (0,n,ubar),
+// the same matrix whose action on dQ is roe_flux's dissipation: two
+// multiply-adds per entry where the product of its factors takes fifteen.
+// With RUP states the columns stay in (rho,u,v,w,p): Mop |A| with Mpr = I
+// (Compute_Dissipation_Matrix_Roe_Optimized, MPFLOW3D/src/Roe_Fluxes.cpp:3185-3199).
 __device__ __forceinline__ void roe_abs_jacobian(const double qL[5], const double qR[5], double nx, double ny,
                                                  double nz, const Flow &f, double Aout[25]) {
     Face L, R;
@@ -381,49 +386,37 @@ __device__ __forceinline__ void roe_abs_jacobian(const double qL[5], const doubl
     double E0, E1, E2;
     if (f.entropy_fix) roe_entropy_fix(L.ubar, L.c, R.ubar, R.c, ubar, c, E0, E1, E2);
     else { E0 = fabs(ubar); E1 = fabs(ubar + c); E2 = fabs(ubar - c); }
-    const double n[3] = {nx, ny, nz};
     const double Es = E1 + E2 - 2.0 * E0, Ed = E1 - E2;
-    // D in RUP variables
-    double D[25];
-    D[0] = E0;
-    for (int j = 0; j < 3; j++) D[1 + j] = 0.5 * rho * Ed / c * n[j];
-    D[4] = Es / (2.0 * c * c);
-    for (int k = 0; k < 3; k++) {
-        D[5 * (k + 1) + 0] = 0.0;
-        for (int j = 0; j < 3; j++) D[5 * (k + 1) + 1 + j] = (k == j ? E0 : 0.0) + 0.5 * n[k] * n[j] * Es;
-        D[5 * (k + 1) + 4] = n[k] * Ed / (2.0 * rho * c);
-    }
-    D[20] = 0.0;
-    for (int j = 0; j < 3; j++) D[21 + j] = 0.5 * rho * c * Ed * n[j];
-    D[24] = 0.5 * (E1 + E2);
-    // M^-1 = dq_RUP/dQ_cons (Compute_Transformation_RUP_To_Conservative, Material.cpp:1240-1300);
-    // with RUP states the columns stay in (rho,u,v,w,p): Mop |A| with Mpr = I
-    // (Compute_Dissipation_Matrix_Roe_Optimized, MPFLOW3D/src/Roe_Fluxes.cpp:3185-3199)
-    const double ri = 1.0 / rho, phi = 0.5 * f.gm1 * q2;
-    double DM[25];
+    const double ci = 1.0 / c, hs = 0.5 * Es, hd = 0.5 * Ed * ci;
+    // columns of the two rank-one terms: coefficients of l_p, and of rho l_u
+    double lp[5], lu[5], X[5], Y[5];
     if (f.rup) {
-        for (int k = 0; k < 25; k++) DM[k] = D[k];
+        lp[0] = lp[1] = lp[2] = lp[3] = 0.0;
+        lp[4] = 1.0;
+        lu[0] = lu[4] = 0.0;
+        lu[1] = rho * nx; lu[2] = rho * ny; lu[3] = rho * nz;
     } else {
-        double Mi[25] = {1.0, 0.0, 0.0, 0.0, 0.0,
-                         -u * ri, ri, 0.0, 0.0, 0.0,
-                         -v * ri, 0.0, ri, 0.0, 0.0,
-                         -w * ri, 0.0, 0.0, ri, 0.0,
-                         phi, -u * f.gm1, -v * f.gm1, -w * f.gm1, f.gm1};
-        for (int i = 0; i < 5; i++)
-            for (int j = 0; j < 5; j++) {
-                double s = 0.0;
-                for (int k = 0; k < 5; k++) s += D[5 * i + k] * Mi[5 * k + j];
-                DM[5 * i + j] = s;
-            }
+        lp[0] = 0.5 * f.gm1 * q2; lp[1] = -f.gm1 * u; lp[2] = -f.gm1 * v; lp[3] = -f.gm1 * w; lp[4] = f.gm1;
+        lu[0] = -ubar; lu[1] = nx; lu[2] = ny; lu[3] = nz; lu[4] = 0.0;
     }
-    // M = dQ_cons/dq_RUP
+    const double hc = hs * ci * ci;
+#pragma unroll
     for (int j = 0; j < 5; j++) {
-        const double d0 = DM[j], d1 = DM[5 + j], d2 = DM[10 + j], d3 = DM[15 + j], d4 = DM[20 + j];
-        Aout[j] = d0;
-        Aout[5 + j] = u * d0 + rho * d1;
-        Aout[10 + j] = v * d0 + rho * d2;
-        Aout[15 + j] = w * d0 + rho * d3;
-        Aout[20 + j] = (phi / f.gm1) * d0 + rho * (u * d1 + v * d2 + w * d3) + d4 / f.gm1;
+        X[j] = hc * lp[j] + hd * lu[j];
+        Y[j] = hs * lu[j] + hd * lp[j];
+    }
+    if (f.rup) dcons_drup(rho, u, v, w, f, Aout);
+#pragma unroll
+    for (int j = 0; j < 5; j++) {
+        auto at = [&](int i, double r, double t) {
+            const double e = f.rup ? E0 * Aout[5 * i + j] : (i == j ? E0 : 0.0);
+            Aout[5 * i + j] = e + r * X[j] + t * Y[j];
+        };
+        at(0, 1.0, 0.0);
+        at(1, u, nx);
+        at(2, v, ny);
+        at(3, w, nz);
+        at(4, ht, ubar);
     }
 }
 
