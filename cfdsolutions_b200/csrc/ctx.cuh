@@ -199,6 +199,7 @@ struct SpmvBatch {
 };
 // keys of the fused SpMV launches: kSpmvKey + CFD_PREC_FP64 / FP32 / BF16
 constexpr int kSpmvKey = 64;
+int spmv_blocks(int nrow);  // CTAs of a job
 int launch_spmv_batch(int key, const SpmvBatch &b, cudaStream_t s);
 }  // namespace cfd
 

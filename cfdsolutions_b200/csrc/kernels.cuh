@@ -286,6 +286,7 @@ __device__ __forceinline__ void store_low(uint16_t *p, double v) {
     __nv_bfloat16 b = __double2bfloat16(v);
     *p = *reinterpret_cast<uint16_t *>(&b);
 }
+__device__ __forceinline__ double load_low(const double *p) { return *p; }
 __device__ __forceinline__ double load_low(const float *p) { return (double)*p; }
 __device__ __forceinline__ double load_low(const uint16_t *p) {
     __nv_bfloat16 b = *reinterpret_cast<const __nv_bfloat16 *>(p);

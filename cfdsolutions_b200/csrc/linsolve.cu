@@ -363,15 +363,19 @@ __global__ void k_sub(int64_t n, const double *__restrict__ b, const double *__r
 
 // ----------------------------------------------------------- block SpMV
 // y_i = sum_k A_k x_{JA[k]}, FP64 accumulation whatever the storage type.
-// Five lanes per block row, lane m forming output m from row m of each 5x5
-// block: the five lanes of a row read its 100-byte FP32 block together, and a
-// warp covers 6.4 consecutive rows, whose blocks are consecutive in memory.
-// Two blocks per step with their own partial sums (even and odd blocks of the
-// row, added at the end) keep twice the loads in flight.  Measured at 128^3
-// (2.15 M rows, 31.8 M blocks, FP32): 0.78 ms, 4.46 TB/s of algorithmic
-// traffic; one warp per row (lane = block element, contiguous 100-byte block
-// loads) reached only 1.7-2.3 TB/s, staging the row through shared memory
-// 3.1 TB/s: fewer bytes in flight per warp.
+// Five lanes per block row, six rows per warp (lanes 30 and 31 idle), lane c
+// multiplying column c of each 5x5 block: a block costs a lane one value of x
+// and five entries of A, each load of five lanes contiguous, where a lane that
+// owns an output loads all five values of x and a strided row of the block.
+// Five blocks are in flight per lane; the column ids are loaded two such
+// batches ahead and the values of x one ahead, so that no load waits for
+// another one.  The partial outputs are added across the five lanes through
+// shared memory at the end of the row.
+// Measured on the 96^3 cube (0.91 M rows, 13.5 M blocks), of 6.45 TB/s: FP32
+// 281 us, 5.3 TB/s (336 us with a lane per output; 320 without the ids and
+// values ahead), FP64 436 us, 6.4 TB/s (482): bound by DRAM.  Slower: the CTA's
+// blocks staged in shared memory by 16-byte copies (320-348 us, FP32: fewer
+// warps), prefetching a later CTA's blocks into L2 (379 us).
 template <typename TA>
 __device__ __forceinline__ double ldA(const TA *p);
 template <>
@@ -381,67 +385,90 @@ __device__ __forceinline__ double ldA<float>(const float *p) { return (double)__
 template <>
 __device__ __forceinline__ double ldA<uint16_t>(const uint16_t *p) { return load_low(p); }
 
-// thread t of a block SpMV: row t/5, component t%5
+constexpr int kSpmvWarps = 4, kSpmvRows = 6 * kSpmvWarps, kSpmvThreads = 32 * kSpmvWarps;
+// The block SpMV of rows kSpmvRows * cta .. of one CTA.
 template <typename TA>
-__device__ __forceinline__ void bspmv_thread(int t, int nrow, const int *__restrict__ IA, const int *__restrict__ JA,
-                                             const TA *__restrict__ A, const double *__restrict__ x,
-                                             double *__restrict__ y) {
-    const int r = t / 5, m = t - 5 * r;
-    if (r >= nrow) return;
-    double s0 = 0.0, s1 = 0.0;
-    int k = IA[r];
-    const int k1 = IA[r + 1];
-    for (; k + 1 < k1; k += 2) {
-        const TA *a = A + (int64_t)k * 25 + m * 5;
-        const double *xv = x + (int64_t)JA[k] * 5, *xw = x + (int64_t)JA[k + 1] * 5;
-        double av[10];
+__device__ __forceinline__ void bspmv_cta(int cta, int nrow, const int *__restrict__ IA, const int *__restrict__ JA,
+                                          const TA *__restrict__ A, const double *__restrict__ x,
+                                          double *__restrict__ y) {
+    __shared__ double part[kSpmvWarps][32 * 5];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int g = lane / 5, c = lane - 5 * g;
+    const int r = cta * kSpmvRows + 6 * w + g;
+    const bool on = lane < 30 && r < nrow;
+    double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    if (on) {
+        const unsigned group = 31u << (5 * g);
+        int k = IA[r];
+        const int k1 = IA[r + 1];
+        const TA *a = A + (int64_t)k * 25 + c;
+        // column ids two batches of five blocks ahead, values of x one ahead
+        auto ids = [&](int at) { return at + c < k1 ? JA[at + c] : 0; };
+        auto values = [&](int j, double v[5]) {
 #pragma unroll
-        for (int q = 0; q < 5; q++) {
-            av[q] = ldA<TA>(a + q);
-            av[5 + q] = ldA<TA>(a + 25 + q);
+            for (int t = 0; t < 5; t++) v[t] = __ldg(x + (int64_t)__shfl_sync(group, j, 5 * g + t) * 5 + c);
+        };
+        double xv[5];
+        int j1 = ids(k), j2 = ids(k + 5);
+        values(j1, xv);
+        for (; k + 5 <= k1; k += 5, a += 125) {
+            double av[25], xn[5];
+#pragma unroll
+            for (int t = 0; t < 25; t++) av[t] = load_low(a + 5 * t);
+            values(j2, xn);
+            j2 = ids(k + 10);
+#pragma unroll
+            for (int t = 0; t < 5; t++)
+#pragma unroll
+                for (int m = 0; m < 5; m++) acc[m] = fma(av[5 * t + m], xv[t], acc[m]);
+#pragma unroll
+            for (int t = 0; t < 5; t++) xv[t] = xn[t];
         }
 #pragma unroll
-        for (int q = 0; q < 5; q++) {
-            s0 = fma(av[q], __ldg(xv + q), s0);
-            s1 = fma(av[5 + q], __ldg(xw + q), s1);
-        }
-    }
-    if (k < k1) {
-        const TA *a = A + (int64_t)k * 25 + m * 5;
-        const double *xv = x + (int64_t)JA[k] * 5;
+        for (int t = 0; t < 4; t++)
+            if (k + t < k1) {
 #pragma unroll
-        for (int q = 0; q < 5; q++) s0 = fma(ldA<TA>(a + q), __ldg(xv + q), s0);
+                for (int m = 0; m < 5; m++) acc[m] = fma(load_low(a + 25 * t + 5 * m), xv[t], acc[m]);
+            }
     }
-    y[(int64_t)r * 5 + m] = s0 + s1;
+    double *p = part[w];
+#pragma unroll
+    for (int m = 0; m < 5; m++) p[5 * lane + m] = acc[m];
+    __syncwarp();
+    if (on) {
+        p += 25 * g + c;
+        y[(int64_t)r * 5 + c] = ((p[0] + p[5]) + (p[10] + p[15])) + p[20];
+    }
 }
 
 template <typename TA>
-__global__ void __launch_bounds__(160) k_bspmv(int nrow, const int *__restrict__ IA, const int *__restrict__ JA,
-                                               const TA *__restrict__ A, const double *__restrict__ x,
-                                               double *__restrict__ y) {
-    bspmv_thread<TA>(blockIdx.x * blockDim.x + threadIdx.x, nrow, IA, JA, A, x, y);
+__global__ void __launch_bounds__(kSpmvThreads) k_bspmv(int nrow, const int *__restrict__ IA, const int *__restrict__ JA,
+                                                        const TA *__restrict__ A, const double *__restrict__ x,
+                                                        double *__restrict__ y) {
+    bspmv_cta<TA>((int)blockIdx.x, nrow, IA, JA, A, x, y);
 }
 
 // Several requests' SpMVs in one launch (the serving loop's fused SpMV): CTA
 // b belongs to the job whose [block_begin, next block_begin) holds it, and
 // computes that job's rows exactly as k_bspmv's CTA b - block_begin would.
 template <typename TA>
-__global__ void __launch_bounds__(160) k_bspmv_batch(const __grid_constant__ SpmvBatch B) {
+__global__ void __launch_bounds__(kSpmvThreads) k_bspmv_batch(const __grid_constant__ SpmvBatch B) {
     int j = 0;
     while (j + 1 < B.njobs && (int)blockIdx.x >= B.job[j + 1].block_begin) j++;
     const SpmvJob &J = B.job[j];
-    bspmv_thread<TA>(((int)blockIdx.x - J.block_begin) * 160 + (int)threadIdx.x, J.nrow, J.IA, J.JA,
-                     static_cast<const TA *>(J.A), J.x, J.y);
+    bspmv_cta<TA>((int)blockIdx.x - J.block_begin, J.nrow, J.IA, J.JA, static_cast<const TA *>(J.A), J.x, J.y);
 }
+
+int spmv_blocks(int nrow) { return grid_for(nrow, kSpmvRows); }
 
 int launch_spmv_batch(int key, const SpmvBatch &b, cudaStream_t s) {
     int blocks = 0;
-    for (int k = 0; k < b.njobs; k++) blocks += grid_for(5 * (int64_t)b.job[k].nrow, 160);
+    for (int k = 0; k < b.njobs; k++) blocks += spmv_blocks(b.job[k].nrow);
     if (blocks == 0) return CFD_OK;
     switch (key - kSpmvKey) {
-        case CFD_PREC_FP64: k_bspmv_batch<double><<<blocks, 160, 0, s>>>(b); break;
-        case CFD_PREC_FP32: k_bspmv_batch<float><<<blocks, 160, 0, s>>>(b); break;
-        case CFD_PREC_BF16: k_bspmv_batch<uint16_t><<<blocks, 160, 0, s>>>(b); break;
+        case CFD_PREC_FP64: k_bspmv_batch<double><<<blocks, kSpmvThreads, 0, s>>>(b); break;
+        case CFD_PREC_FP32: k_bspmv_batch<float><<<blocks, kSpmvThreads, 0, s>>>(b); break;
+        case CFD_PREC_BF16: k_bspmv_batch<uint16_t><<<blocks, kSpmvThreads, 0, s>>>(b); break;
         default: return CFD_ERR_UNSUPPORTED;
     }
     CFD_LAUNCH_CHECK();
@@ -754,7 +781,7 @@ static int precond_apply(cfd_ctx *c, const Precond &pc, const double *r, double 
 
 static int spmv(cfd_ctx *c, int prec, const double *x, double *y) {
     const int n = c->nnode;
-    const int g = grid_for(5 * (int64_t)n, 160), b = 160;
+    const int g = spmv_blocks(n), b = kSpmvThreads;
     if (prec == CFD_PREC_FP64 && !c->a64_valid) prec = c->a_precision;  // low-precision-only system
     const void *A = prec == CFD_PREC_FP32 && c->A32.p   ? (const void *)c->A32.p
                     : prec == CFD_PREC_BF16 && c->A16.p ? (const void *)c->A16.p

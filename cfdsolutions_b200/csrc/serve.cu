@@ -113,7 +113,7 @@ struct Batcher {
             for (int k = 0; k < b.njobs; k++) {
                 b.job[k] = take[k]->spmv;
                 b.job[k].block_begin = blk;
-                blk += (int)((5 * (int64_t)b.job[k].nrow + 159) / 160);
+                blk += cfd::spmv_blocks(b.job[k].nrow);
             }
             return cfd::launch_spmv_batch(key, b, s);
         }
