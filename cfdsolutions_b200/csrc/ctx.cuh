@@ -86,17 +86,19 @@ struct Levels {
 // a colour.
 struct Abmc {
     bool built = false;
-    int ncolor = 0, maxrow = 0, maxstage = 0;
+    int ncolor = 0, maxrow = 0, maxstage = 0, maxblk = 0, maxpairs = 0, stage = 0;
+    bool by_cta = false;              // patches fit the CTA-per-patch factorisation
     std::vector<int> cptr;            // host [ncolor+1] into patches
     std::vector<int> h_pcolor;        // host colour of each patch
     DevBuf<int> patches;              // patch ids in colour order
     DevBuf<int> slot;                 // [nnzb] per row: lower slots (factorisation order) | diag | upper slots
-    DevBuf<int4> meta;                // per row: external lower, lower, intra-patch upper, 0
-    DevBuf<unsigned> loc;             // [nnzb] place of each slot entry's factor block in M
+    DevBuf<int4> meta;                // per row: external lower, lower, intra-patch upper, level in the patch |
+                                      // pairs of its external lower blocks << 8
+    DevBuf<unsigned> loc;             // [nnzb] place of each CRS block's factor in M
     int64_t nelem = 0;                // elements of M
-    DevBuf<int4> hdr;                 // [nnzb] per lower block: place of inv(U_pp) in M, pairs, local slot
+    DevBuf<int4> hdr;                 // [nnzb] per lower block: inv(U_pp), pairs, local slot, level (see k_mc_factor)
     DevBuf<int64_t> pair_ptr;         // [n+1] update pairs of each row
-    DevBuf<int2> pairs;               // (place of U_pj in M, local slot of (i,j))
+    DevBuf<int2> pairs;               // (U_pj, local slot of (i,j))
     // triangular solves (0 forward, 1 backward), patches in launch order: per
     // patch {first 16-byte word of its lists, words, first unit of its region
     // of M, units}; per colour the largest {words, units, columns, elements before the slots}

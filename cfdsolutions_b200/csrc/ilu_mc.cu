@@ -69,29 +69,35 @@ __device__ __forceinline__ bool warp_inverse5(double &a, double &v, int lane) {
     bool ok = true;
 #pragma unroll
     for (int k = 0; k < 5; k++) {
-        // pivot: largest |a(r,k)| over r >= k, lowest r on ties
-        double best = (on && c == k && r >= k) ? fabs(a) : -1.0;
-        int brow = r;
+        // column k, on every lane; pivot: its largest magnitude at or below
+        // row k, lowest row on ties.  Every lane inverts its own entry
+        // meanwhile: the pivot's is among them.
+        const double inv_own = 1.0 / a;
+        double col[5];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-            const int orow = __shfl_xor_sync(0xffffffffu, brow, o);
-            if (ob > best || (ob == best && orow < brow)) { best = ob; brow = orow; }
+        for (int t = 0; t < 5; t++) col[t] = __shfl_sync(0xffffffffu, a, t * 5 + k);
+        int p = k;
+        double pv = col[k];
+#pragma unroll
+        for (int t = k + 1; t < 5; t++)
+            if (fabs(col[t]) > fabs(pv)) { pv = col[t]; p = t; }
+        if (!(fabs(pv) > 0.0)) ok = false;
+        // rows k and p change places; row k is scaled by 1 / pivot and
+        // eliminated from the others
+        const double d = __shfl_sync(0xffffffffu, inv_own, p * 5 + k);
+        const double ak = __shfl_sync(0xffffffffu, a, p * 5 + (on ? c : 0)) * d;
+        const double vk = __shfl_sync(0xffffffffu, v, p * 5 + (on ? c : 0)) * d;
+        const double a0 = __shfl_sync(0xffffffffu, a, k * 5 + (on ? c : 0));
+        const double v0 = __shfl_sync(0xffffffffu, v, k * 5 + (on ? c : 0));
+        double f = 0.0;
+#pragma unroll
+        for (int t = 0; t < 5; t++)
+            if (t == r) f = col[t];
+        if (r == p) { f = col[k]; a = a0; v = v0; }
+        if (on) {
+            a = r == k ? ak : a - f * ak;
+            v = r == k ? vk : v - f * vk;
         }
-        if (!(best > 0.0)) ok = false;
-        // swap rows k and brow
-        const int sr = r == k ? brow : (r == brow ? k : r);
-        const int from = on ? sr * 5 + c : lane;
-        a = __shfl_sync(0xffffffffu, a, from);
-        v = __shfl_sync(0xffffffffu, v, from);
-        // scale row k by 1/a(k,k)
-        const double d = 1.0 / __shfl_sync(0xffffffffu, a, k * 5 + k);
-        if (on && r == k) { a *= d; v *= d; }
-        // eliminate column k from the other rows
-        const double f = __shfl_sync(0xffffffffu, a, (on ? r : 0) * 5 + k);
-        const double ak = __shfl_sync(0xffffffffu, a, k * 5 + (on ? c : 0));
-        const double vk = __shfl_sync(0xffffffffu, v, k * 5 + (on ? c : 0));
-        if (on && r != k) { a -= f * ak; v -= f * vk; }
     }
     return ok;
 }
@@ -123,6 +129,41 @@ __device__ __forceinline__ int64_t mc_element(unsigned p, int r, int c) {
     return (int64_t)(p & ~kMcSlotBit) * 5 + k + c;
 }
 
+// One step of a row's elimination by a warp: L_ip = A_ip inv(U_pp) in block tk
+// of w, then A_ij -= L_ip U_pj over the step's cnt pairs, target(t) the block
+// of pair t, inv(k) / U(t, k) entry k of the factor blocks.  Lane 5 r + c owns
+// entry (r, c) of every block; four pairs are in flight (no two have the same
+// target).
+template <typename FT, typename FI, typename FU>
+__device__ __forceinline__ void mc_eliminate(double *w, int tk, int cnt, FT target, FI inv, FU U, int lane) {
+    const int r = min(lane / 5, 4), c = lane - 5 * (lane / 5);
+    const bool on = lane < 25;
+    double *row = w + tk * 25 + 5 * r;
+    double L[5], Lrc = 0.0;
+#pragma unroll
+    for (int k = 0; k < 5; k++) Lrc = fma(row[k], inv(5 * k + c), Lrc);
+    __syncwarp();
+    if (on) row[c] = Lrc;
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 5; k++) L[k] = row[k];
+    for (int t0 = 0; t0 < cnt; t0 += 4) {
+        double *d[4], v[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int t = min(t0 + j, cnt - 1);
+            d[j] = w + target(t) * 25 + (on ? lane : 0);
+            v[j] = *d[j];
+#pragma unroll
+            for (int k = 0; k < 5; k++) v[j] = fma(-L[k], U(t, 5 * k + c), v[j]);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            if (on && t0 + j < cnt) *d[j] = v[j];
+    }
+    __syncwarp();
+}
+
 // Shared-memory bytes of one warp of k_mc_factor (factor blocks staged in
 // their storage type TM), rounded up to 16.
 template <typename TM>
@@ -143,9 +184,11 @@ __host__ __device__ inline size_t mc_factor_warp_bytes(int maxrow, int maxstage)
 // shared memory: for each lower block, in factorisation order,
 // L_ip = A_ip inv(U_pp) and A_ij -= L_ip U_pj over the row's pairs of p.
 // The factors are stored by patch, as the triangular solves stage them:
-// loc[IA[i]+u] is the place of row i's entry u.
-// hdr[IA[i]+u] = (place of inv(U_pp), pairs, CRS-local slot of (i,p));
-// pairs are (place of U_pj, CRS-local slot of (i,j)).
+// loc[k] is the place of CRS block k, meta[i].w = level of row i in its patch |
+// pairs of its off-patch blocks << 8.
+// hdr[IA[i]+u] = (place of inv(U_pp), pairs, CRS-local slot of (i,p), 0);
+// pairs are (place of U_pj, CRS-local slot of (i,j)).  For p in row i's patch
+// the places are CRS positions in the patch instead, and hdr.w is p's level.
 template <typename TA, typename TM>
 __global__ void k_mc_factor(const int *__restrict__ patches, int npatch, int n, int maxrow, int maxstage,
                             const int *__restrict__ IA, const int *__restrict__ slot, const int4 *__restrict__ meta,
@@ -166,7 +209,7 @@ __global__ void k_mc_factor(const int *__restrict__ patches, int npatch, int n, 
     const int pidx = blockIdx.x * nwarp + wid;
     if (pidx >= npatch) return;  // whole warp; no CTA barrier follows
     const int P = patches[pidx];
-    const int p0 = P * kMcRows, nr = min(kMcRows, n - p0);
+    const int p0 = P * kMcRows, nr = min(kMcRows, n - p0), base0 = IA[p0];
     const int a = lane / 5, b = lane - 5 * (lane / 5);
     {
         for (int q = 0; q < nr; q++) {
@@ -174,16 +217,17 @@ __global__ void k_mc_factor(const int *__restrict__ patches, int npatch, int n, 
             const int4 mt = meta[i];
             const int base = IA[i], len = IA[i + 1] - base, nlo = mt.y;
             const int64_t pp = pair_ptr[i];
-            const int npair = (int)(pair_ptr[i + 1] - pp);
+            const int npair = (int)(pair_ptr[i + 1] - pp), next_pairs = mt.w >> 8;
             for (int e = lane; e < nlo; e += 32) {
                 const int4 h = hdr[base + e];
                 hd[e] = h;
-                src[e] = h.x;
+                // blocks of the patch's own rows are named by their position in it
+                src[e] = e < mt.x ? h.x : (int)loc[base0 + h.x];
             }
             for (int e = lane; e < npair; e += 32) {
                 const int2 pr = pairs[pp + e];
                 pm[e] = pr.y;
-                src[nlo + e] = pr.x;
+                src[nlo + e] = e < next_pairs ? pr.x : (int)loc[base0 + pr.x];
             }
             for (int e = lane; e < len; e += 32) sl[e] = slot[base + e] - base;
             // one block per lane, its 25 loads in flight together
@@ -194,36 +238,24 @@ __global__ void k_mc_factor(const int *__restrict__ patches, int npatch, int n, 
             }
             __syncwarp();
             const int nst = nlo + npair;
-            for (int t = lane; t < nst; t += 32) {
-                const unsigned p = (unsigned)src[t];
+            // a block per step, an entry per lane, eight steps in flight
+            for (int t8 = 0; t8 < nst; t8 += 8) {
+                TM v[8];
 #pragma unroll
-                for (int k = 0; k < 25; k++) stg[t * 25 + k] = M[mc_element(p, k / 5, k % 5)];
+                for (int k = 0; k < 8; k++)
+                    v[k] = M[mc_element((unsigned)src[min(t8 + k, nst - 1)], min(a, 4), b)];
+#pragma unroll
+                for (int k = 0; k < 8; k++)
+                    if (t8 + k < nst && lane < 25) stg[(t8 + k) * 25 + lane] = v[k];
             }
             __syncwarp();
             int t0 = 0;
             for (int u = 0; u < nlo; u++) {
                 const int4 h = hd[u];
-                const int tk = h.z;
-                // L_ip = A_ip inv(U_pp)
-                double Lab = 0.0;
-                if (lane < 25) {
-#pragma unroll
-                    for (int c = 0; c < 5; c++) Lab = fma(w[tk * 25 + a * 5 + c], (double)stg[u * 25 + c * 5 + b], Lab);
-                }
-                __syncwarp();
-                if (lane < 25) w[tk * 25 + lane] = Lab;
-                __syncwarp();
-                // A_ij -= L_ip U_pj, the pairs' 25 entries spread over the lanes
-                for (int e = lane; e < h.y * 25; e += 32) {
-                    const int t = e / 25, ab = e - 25 * t, ea = ab / 5, eb = ab - 5 * ea;
-                    const int mj = pm[t0 + t];
-                    const TM *U = stg + (size_t)(nlo + t0 + t) * 25;
-                    double s = w[mj * 25 + ab];
-#pragma unroll
-                    for (int c = 0; c < 5; c++) s = fma(-w[tk * 25 + ea * 5 + c], (double)U[c * 5 + eb], s);
-                    w[mj * 25 + ab] = s;
-                }
-                __syncwarp();
+                const TM *iv = stg + u * 25, *Up = stg + (size_t)(nlo + t0) * 25;
+                const int *to = pm + t0;
+                mc_eliminate(w, h.z, h.y, [&](int t) { return to[t]; }, [&](int k) { return (double)iv[k]; },
+                             [&](int t, int k) { return (double)Up[t * 25 + k]; }, lane);
                 t0 += h.y;
             }
             const int td = sl[nlo];  // the diagonal follows the lower entries
@@ -237,11 +269,206 @@ __global__ void k_mc_factor(const int *__restrict__ patches, int npatch, int n, 
             __syncwarp();
             for (int e = lane; e < len * 25; e += 32) {
                 const int u = e / 25, rc = e - 25 * u;
-                st<TM>(M + mc_element(loc[base + u], rc / 5, rc % 5), w[sl[u] * 25 + rc]);
+                st<TM>(M + mc_element(loc[base + sl[u]], rc / 5, rc % 5), w[sl[u] * 25 + rc]);
             }
             __syncwarp();
         }
     }
+}
+
+// Factorisation of the patches of one colour, one CTA of 16 warps per patch:
+// the same operations as the warp-per-patch kernel, for meshes whose patches'
+// blocks fit in shared memory in FP64.  The patch's blocks and lists are
+// loaded once.  Blocks that couple to other patches come first in every row's
+// order and depend on nothing inside the patch, so the warps, two rows each,
+// eliminate them at once, staging the factor blocks of the other patches.
+// Then, level by level, the rows of a level invert their diagonal blocks, and
+// every row eliminates its blocks in their columns.
+// Bound by the chain of a patch's levels, some 9 inversions and eliminations
+// behind each other, where the warp-per-patch kernel takes 32 rows one after
+// the other.  A cfd_gmres call of one iteration (factorisation, two applies) on
+// the tet cubes, FP32 / FP64: 24^3 0.91 / 0.98 ms, 48^3 2.1 / 2.3, 64^3 4.0 /
+// 4.4, 96^3 11.5 / 12.8; with the warp-per-patch kernel 4.0 / 4.6, 5.2 / 5.8,
+// 6.5 / 7.4 and 12.6 / 15.4 ms.
+constexpr int kMcFactorWarps = 16, kMcFactorRows = kMcRows / kMcFactorWarps;
+static_assert(kMcFactorRows == 2, "two rows per warp");
+constexpr size_t kMcFactorBytes = 222u << 10;  // its shared memory at most
+__host__ __device__ inline size_t mc_factor_cta_bytes(int maxblk, int maxpairs) {
+    return ((size_t)maxblk * (25 * sizeof(double) + sizeof(int4) + 2 * sizeof(int)) + (size_t)maxpairs * sizeof(int2) + 15) &
+           ~(size_t)15;
+}
+
+template <typename TA, typename TM>
+__global__ void __launch_bounds__(32 * kMcFactorWarps, 1) k_mc_factor_cta(
+    const int *__restrict__ patches, int n, int maxblk, int maxpairs, int stage, const int *__restrict__ IA,
+    const int *__restrict__ slot, const int4 *__restrict__ meta, const int4 *__restrict__ hdr,
+    const unsigned *__restrict__ loc, const int64_t *__restrict__ pair_ptr, const int2 *__restrict__ pairs,
+    const TA *__restrict__ A, TM *__restrict__ M, int *__restrict__ err) {
+    extern __shared__ __align__(16) unsigned char smraw[];
+    __shared__ int4 mts[kMcRows];                          // the rows' meta
+    __shared__ int first[kMcRows + 1], pfirst[kMcRows + 1];  // first block / pair of each row in the patch
+    int4 *hd = reinterpret_cast<int4 *>(smraw);                          // [maxblk]
+    double *w = reinterpret_cast<double *>(hd + maxblk);                 // [maxblk][25], CRS slot order
+    int2 *pr = reinterpret_cast<int2 *>(w + (size_t)maxblk * 25);        // [maxpairs]
+    int *sl = reinterpret_cast<int *>(pr + maxpairs);                    // [maxblk] CRS position of list entry u
+    unsigned *at = reinterpret_cast<unsigned *>(sl + maxblk);            // [maxblk] place in M of CRS position k
+    constexpr int NT = 32 * kMcFactorWarps;
+    const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
+    TM *stg = reinterpret_cast<TM *>(smraw + mc_factor_cta_bytes(maxblk, maxpairs)) + (size_t)wid * stage * 25;
+    const int p0 = patches[blockIdx.x] * kMcRows, nr = min(kMcRows, n - p0);
+    const int base = IA[p0], nblk = IA[p0 + nr] - base;
+    const int64_t pbase = pair_ptr[p0];
+    const int npair = (int)(pair_ptr[p0 + nr] - pbase);
+    const TA *Ap = A + (int64_t)base * 25;
+    for (int e0 = tid; e0 < nblk * 25; e0 += 8 * NT) {
+        double v[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) v[k] = ld<TA>(Ap + min(e0 + k * NT, nblk * 25 - 1));
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+            if (e0 + k * NT < nblk * 25) w[e0 + k * NT] = v[k];
+    }
+    for (int e = tid; e <= nr; e += NT) {
+        first[e] = IA[p0 + e] - base;
+        pfirst[e] = (int)(pair_ptr[p0 + e] - pbase);
+        if (e < nr) mts[e] = meta[p0 + e];
+    }
+    for (int e = tid; e < nblk; e += NT) {
+        hd[e] = hdr[base + e];
+        sl[e] = slot[base + e] - base;
+        at[e] = loc[base + e];
+    }
+    for (int e = tid; e < npair; e += NT) pr[e] = pairs[pbase + e];
+    __syncthreads();
+    const int a = min(lane / 5, 4), b = lane - 5 * (lane / 5);
+    // rows to warps in order of their levels, so that a level's rows have
+    // different warps
+    const int mylev = lane < nr ? mts[lane].w & 255 : -1;
+    int last = 0, rank = 0, before = 0;
+    for (int l = 0; before < nr && l < kMcRows; l++) {
+        const unsigned m = __ballot_sync(0xffffffffu, mylev == l);
+        if (mylev == l) rank = before + __popc(m & ((1u << lane) - 1u));
+        before += __popc(m);
+        last = l;
+    }
+    int rows[kMcFactorRows];  // the warp's rows, nr: none
+#pragma unroll
+    for (int k = 0; k < kMcFactorRows; k++) {
+        const unsigned m = __ballot_sync(0xffffffffu, lane < nr && rank == wid + k * kMcFactorWarps);
+        rows[k] = m ? __ffs(m) - 1 : nr;
+    }
+    // blocks that couple to other patches: as many at a time as the staging holds
+#pragma unroll 1
+    for (int k = 0; k < kMcFactorRows; k++) {
+        const int q = k == 0 ? rows[0] : rows[1];
+        if (q >= nr) continue;
+        const int row0 = first[q], next = mts[q].x;
+        const int2 *q0 = pr + pfirst[q];
+        for (int u0 = 0; u0 < next;) {
+            int u1 = u0, np = 0;
+            for (; u1 < next; u1++) {
+                const int y = hd[row0 + u1].y;
+                if (u1 > u0 && u1 + 1 - u0 + np + y > stage) break;
+                np += y;
+            }
+            const int m = u1 - u0 + np;
+            // a block per step, an entry per lane, eight steps in flight
+            for (int t8 = 0; t8 < m; t8 += 8) {
+                TM v[8];
+#pragma unroll
+                for (int k = 0; k < 8; k++) {
+                    const int t = min(t8 + k, m - 1);
+                    const unsigned p = (unsigned)(t < u1 - u0 ? hd[row0 + u0 + t].x : q0[t - (u1 - u0)].x);
+                    v[k] = M[mc_element(p, a, b)];
+                }
+#pragma unroll
+                for (int k = 0; k < 8; k++)
+                    if (t8 + k < m && lane < 25) stg[(t8 + k) * 25 + lane] = v[k];
+            }
+            __syncwarp();
+            const TM *Up = stg + (u1 - u0) * 25;
+            for (int u = u0; u < u1; u++) {
+                const int4 h = hd[row0 + u];
+                const TM *iv = stg + (u - u0) * 25;
+                mc_eliminate(w, row0 + h.z, h.y, [&](int t) { return row0 + q0[t].y; },
+                             [&](int k) { return (double)iv[k]; }, [&](int t, int k) { return (double)Up[t * 25 + k]; },
+                             lane);
+                q0 += h.y;
+                Up += h.y * 25;
+            }
+            u0 = u1;
+        }
+    }
+    // the headers of the warp's rows' intra-patch blocks, one per lane, with
+    // the place of their pairs (a row has at most 31 of them)
+    int4 mine[kMcFactorRows];
+    int pairs_at[kMcFactorRows], lev[kMcFactorRows], nin[kMcFactorRows];
+#pragma unroll
+    for (int k = 0; k < kMcFactorRows; k++) {
+        const int q = rows[k];
+        lev[k] = -1;
+        nin[k] = 0;
+        mine[k] = make_int4(0, 0, 0, -1);
+        if (q < nr) {
+            lev[k] = mts[q].w & 255;
+            nin[k] = mts[q].y - mts[q].x;
+            if (lane < nin[k]) mine[k] = hd[first[q] + mts[q].x + lane];
+        }
+        int sum = mine[k].y;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, sum, o);
+            if (lane >= o) sum += v;
+        }
+        pairs_at[k] = sum - mine[k].y + (q < nr ? pfirst[q] + (mts[q].w >> 8) : 0);
+    }
+    for (int l = 0; l <= last; l++) {
+#pragma unroll
+        for (int k = 0; k < kMcFactorRows; k++) {
+            if (lev[k] != l) continue;
+            const int q = rows[k];
+            double *dg = w + sl[first[q] + mts[q].y] * 25;  // the diagonal follows the lower entries
+            double av = lane < 25 ? dg[lane] : 0.0, iv;
+            const bool ok = warp_inverse5(av, iv, lane);
+            if (!ok && lane == 0) atomicOr(err, ERR_NAN);
+            __syncwarp();
+            if (lane < 25) dg[lane] = iv;
+            __syncwarp();
+            // the other rows see the factors as stored
+            if (sizeof(TM) < sizeof(double)) {
+                const int end = first[q + 1] * 25;
+                for (int e0 = first[q] * 25 + lane; e0 < end; e0 += 256) {
+                    double v[8];
+#pragma unroll
+                    for (int j = 0; j < 8; j++) v[j] = (double)(TM)w[min(e0 + 32 * j, end - 1)];
+#pragma unroll
+                    for (int j = 0; j < 8; j++)
+                        if (e0 + 32 * j < end) w[e0 + 32 * j] = v[j];
+                }
+            }
+        }
+        if (l == last) break;
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kMcFactorRows; k++) {
+            unsigned todo = __ballot_sync(0xffffffffu, lane < nin[k] && mine[k].w == l);
+            const int row0 = first[rows[k]];
+            for (; todo; todo &= todo - 1) {
+                const int s = __ffs(todo) - 1;
+                const int x = __shfl_sync(0xffffffffu, mine[k].x, s), cnt = __shfl_sync(0xffffffffu, mine[k].y, s);
+                const int z = __shfl_sync(0xffffffffu, mine[k].z, s), pa = __shfl_sync(0xffffffffu, pairs_at[k], s);
+                const int2 *q = pr + pa;
+                const double *iv = w + x * 25;
+                mc_eliminate(w, row0 + z, cnt, [&](int t) { return row0 + q[t].y; }, [&](int j) { return iv[j]; },
+                             [&](int t, int j) { return w[q[t].x * 25 + j]; }, lane);
+            }
+        }
+    }
+    __syncthreads();
+    // a block per warp and step, an entry per lane
+#pragma unroll 4
+    for (int k = wid; k < nblk; k += kMcFactorWarps)
+        if (lane < 25) st<TM>(M + mc_element(at[k], a, b), w[k * 25 + lane]);
 }
 
 // Programmatic dependent launch (sm_90+): the solve of one colour lets the
@@ -672,6 +899,17 @@ int mc_build(cfd_ctx *c) {
     parallel_ranges(c->nnzb, [&](int, int64_t u0, int64_t u1) {
         for (int64_t u = u0; u < u1; u++) scol[u] = JA[slot[u]];
     });
+    // A row's level in its patch: the longest chain of intra-patch lower blocks
+    // before it (meta.w, for the factorisation)
+    parallel_patches([&](int, int64_t q0, int64_t q1) {
+        for (int i = (int)q0 * kMcRows; i < std::min<int64_t>(n, q1 * kMcRows); i++) {
+            int l = 0;
+            for (int u = IA[i] + meta[i].x; u < IA[i] + meta[i].y; u++) l = std::max(l, meta[scol[u]].w + 1);
+            meta[i].w = l;
+        }
+    });
+    int maxblk = 0;
+    for (int P = 0; P < np; P++) maxblk = std::max(maxblk, IA[std::min(n, (P + 1) * kMcRows)] - IA[P * kMcRows]);
     // The solves' plan of each patch and direction (0 forward, 1 backward):
     // rows to groups, the region's size, and the lists (layout at kMcWarpAt);
     // then the regions' places in M, in launch order, and every block's place.
@@ -828,25 +1066,36 @@ int mc_build(cfd_ctx *c) {
     // row p = JA[slot[base+u]] whose column row i holds (its CRS-local slot by
     // binary search, JA rows being sorted).  Counted, then written, per row.
     std::vector<int4> hdr(c->nnzb, make_int4(0, 0, 0, 0));
+    std::vector<int> ext_pairs(n, 0);  // pairs of each row's off-patch blocks
     std::vector<int64_t> pair_ptr(n + 1, 0);
     auto row_pairs = [&](int i, int2 *out) {  // returns the row's pair count; writes them when out != nullptr
         const int base = IA[i], end = IA[i + 1];
         const int nlo = meta[i].y;
-        int total = 0;
+        int total = 0, next_pairs = 0;
         for (int u = 0; u < nlo; u++) {
             const int kk = slot[base + u], p = JA[kk];
+            // blocks of the patch's own rows are named by their CRS position in the patch
+            const bool own = u >= meta[i].x;
+            const int patch0 = IA[i / kMcRows * kMcRows];
             int cnt = 0;
             for (int v = IA[p] + meta[p].y + 1; v < IA[p + 1]; v++) {
                 const int j = scol[v];
                 const int *it = std::lower_bound(&JA[base], &JA[0] + end, j);
                 if (it != &JA[0] + end && *it == j) {
-                    if (out) out[total + cnt] = make_int2((int)loc[v], (int)(it - &JA[base]));
+                    if (out) out[total + cnt] = make_int2(own ? slot[v] - patch0 : (int)loc[v], (int)(it - &JA[base]));
                     cnt++;
                 }
             }
-            if (out) hdr[base + u] = make_int4((int)loc[IA[p] + meta[p].y], cnt, kk - base, 0);
+            if (out) {
+                const int dg = IA[p] + meta[p].y;  // the diagonal's list entry
+                hdr[base + u] = make_int4(own ? slot[dg] - patch0 : (int)loc[dg], cnt, kk - base,
+                                          own ? meta[p].w & 255 : 0);
+                if (!own) next_pairs += cnt;
+            }
             total += cnt;
         }
+        // other threads read the level meanwhile: the counts go in afterwards
+        if (out) ext_pairs[i] = next_pairs;
         return total;
     };
     parallel_ranges(n, [&](int, int64_t i0, int64_t i1) {
@@ -857,16 +1106,34 @@ int mc_build(cfd_ctx *c) {
         maxstage = std::max<int64_t>(maxstage, meta[i].y + pair_ptr[i + 1]);
         pair_ptr[i + 1] += pair_ptr[i];
     }
+    int64_t maxpairs = 1;
+    for (int P = 0; P < np; P++)
+        maxpairs = std::max(maxpairs, pair_ptr[std::min(n, (P + 1) * kMcRows)] - pair_ptr[P * kMcRows]);
     std::vector<int2> pairs(std::max<int64_t>(pair_ptr[n], 1));
     parallel_ranges(n, [&](int, int64_t i0, int64_t i1) {
         for (int i = (int)i0; i < (int)i1; i++) row_pairs(i, pairs.data() + pair_ptr[i]);
     });
+    int maxcnt = 0;
+    for (int i = 0; i < n; i++) {
+        meta[i].w |= ext_pairs[i] << 8;
+        for (int u = IA[i]; u < IA[i] + meta[i].x; u++) maxcnt = std::max(maxcnt, hdr[u].y);
+    }
+    // the CTA-per-patch factorisation, when its patches fit in either precision
+    mc.maxblk = maxblk;
+    mc.maxpairs = (int)std::min<int64_t>(maxpairs, 1 << 24);
+    mc.stage = std::max(24, 1 + maxcnt);
+    mc.by_cta = mc_factor_cta_bytes(mc.maxblk, mc.maxpairs) + (size_t)kMcFactorWarps * mc.stage * 25 * sizeof(double) <=
+                kMcFactorBytes;
     mc.maxrow = maxrow;
     mc.maxstage = maxstage;
     CFD_CUDA(mc.patches.upload(patches.data(), patches.size(), c->stream));
     CFD_CUDA(mc.slot.upload(slot.data(), slot.size(), c->stream));
     CFD_CUDA(mc.meta.upload(meta.data(), meta.size(), c->stream));
-    CFD_CUDA(mc.loc.upload(loc.data(), loc.size(), c->stream));
+    std::vector<unsigned> place(c->nnzb);  // by CRS position
+    parallel_ranges(c->nnzb, [&](int, int64_t u0, int64_t u1) {
+        for (int64_t u = u0; u < u1; u++) place[slot[u]] = loc[u];
+    });
+    CFD_CUDA(mc.loc.upload(place.data(), place.size(), c->stream));
     CFD_CUDA(mc.hdr.upload(hdr.data(), hdr.size(), c->stream));
     CFD_CUDA(mc.pair_ptr.upload(pair_ptr.data(), pair_ptr.size(), c->stream));
     CFD_CUDA(mc.pairs.upload(pairs.data(), (size_t)pair_ptr[n], c->stream));
@@ -880,6 +1147,10 @@ int mc_factor(cfd_ctx *c, const TA *A, TM *M) {
     Abmc &mc = c->mc;
     int st = mc_build(c);
     if (st) return st;
+    CFD_CUDA(allow_max_dynamic_smem(k_mc_solve<TM, false, true>, c->device, nullptr));
+    CFD_CUDA(allow_max_dynamic_smem(k_mc_solve<TM, true, true>, c->device, nullptr));
+    // the slots' empty places read as zeros
+    CFD_CUDA(cudaMemsetAsync(M, 0, (size_t)mc.nelem * sizeof(TM), c->stream));
     // four warps (patches) per CTA, fewer when their staging does not fit in
     // 200 KB; several CTAs share an SM so every SM gets patches
     const size_t per_warp = mc_factor_warp_bytes<TM>(mc.maxrow, mc.maxstage);
@@ -890,21 +1161,24 @@ int mc_factor(cfd_ctx *c, const TA *A, TM *M) {
         return CFD_ERR_RANGE;
     }
     const size_t smem = per_warp * nwarp;
+    const size_t smem_cta = mc_factor_cta_bytes(mc.maxblk, mc.maxpairs) + (size_t)kMcFactorWarps * mc.stage * 25 * sizeof(TM);
     int smax = 0;
     CFD_CUDA(allow_max_dynamic_smem(k_mc_factor<TA, TM>, c->device, &smax));
-    CFD_CUDA(allow_max_dynamic_smem(k_mc_solve<TM, false, true>, c->device, nullptr));
-    CFD_CUDA(allow_max_dynamic_smem(k_mc_solve<TM, true, true>, c->device, nullptr));
     if (smem > (size_t)smax) {
         set_error("ILU(0) multicolour: %zu bytes of shared memory needed, %d available", smem, smax);
         return CFD_ERR_RANGE;
     }
-    // the slots' empty places read as zeros
-    CFD_CUDA(cudaMemsetAsync(M, 0, (size_t)mc.nelem * sizeof(TM), c->stream));
+    CFD_CUDA(allow_max_dynamic_smem(k_mc_factor_cta<TA, TM>, c->device, &smax));
     for (int k = 0; k < mc.ncolor; k++) {
         const int cnt = mc.cptr[k + 1] - mc.cptr[k];
-        k_mc_factor<TA, TM><<<grid_for(cnt, nwarp), 32 * nwarp, smem, c->stream>>>(
-            mc.patches.p + mc.cptr[k], cnt, c->nnode, mc.maxrow, mc.maxstage, c->IA.p, mc.slot.p, mc.meta.p,
-            mc.hdr.p, mc.loc.p, mc.pair_ptr.p, mc.pairs.p, A, M, c->err.p);
+        if (mc.by_cta && smem_cta <= (size_t)smax)
+            k_mc_factor_cta<TA, TM><<<cnt, 32 * kMcFactorWarps, smem_cta, c->stream>>>(
+                mc.patches.p + mc.cptr[k], c->nnode, mc.maxblk, mc.maxpairs, mc.stage, c->IA.p, mc.slot.p, mc.meta.p,
+                mc.hdr.p, mc.loc.p, mc.pair_ptr.p, mc.pairs.p, A, M, c->err.p);
+        else
+            k_mc_factor<TA, TM><<<grid_for(cnt, nwarp), 32 * nwarp, smem, c->stream>>>(
+                mc.patches.p + mc.cptr[k], cnt, c->nnode, mc.maxrow, mc.maxstage, c->IA.p, mc.slot.p, mc.meta.p,
+                mc.hdr.p, mc.loc.p, mc.pair_ptr.p, mc.pairs.p, A, M, c->err.p);
     }
     CFD_LAUNCH_CHECK();
     return CFD_OK;
