@@ -893,6 +893,175 @@ __global__ void __launch_bounds__(128) k_gs_level(int nrows, const int *__restri
     for (int m = 0; m < 5; m++) X[(int64_t)r * 5 + m] = xo[m];
 }
 
+// A whole sweep in one launch: one cluster of kGsCtas CTAs walks the levels,
+// separated by the cluster's hardware barrier, where a launch per level cost
+// 19 us for some hundred rows.  Five lanes per row (six rows per warp), lane m
+// forming component m with k_gs_level's operations in the same order.  What
+// does not depend on X -- a row's blocks, its LU factors and column ids -- is
+// copied to shared memory one chunk of rows ahead, across level bounds; after
+// the barrier one round trip to L2 fetches the values of X.
+constexpr int kGsCtas = 8, kGsWarps = 4, kGsRows = 6 * kGsWarps, kGsThreads = 32 * kGsWarps;
+constexpr int kGsBlocks = 16;  // blocks of a row staged (the rest are read from global memory)
+constexpr int kGsMeanWidth = 2048;  // mean rows per level up to which the cluster sweeps
+struct GsStage {
+    double A[kGsRows][kGsBlocks * 25];
+    double LU[kGsRows][25];
+    int JA[kGsRows][kGsBlocks];
+};
+struct GsShared {
+    GsStage stage[2];
+    double x[kGsRows][kGsBlocks * 5 + 1];
+};
+
+__device__ __forceinline__ void gs_copy8(void *smem, const void *gmem) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem)
+                 : "memory");
+}
+__device__ __forceinline__ void gs_copy4(void *smem, const void *gmem) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem)
+                 : "memory");
+}
+
+// desc[t] = {row, first block, end, diagonal block} in level order; stop[0] != 0: nothing to do
+__global__ void __launch_bounds__(kGsThreads, 1) k_gs_sweep(int nlevels, const int *__restrict__ ptr,
+                                                            const int4 *__restrict__ desc, const int *__restrict__ JA,
+                                                            const double *__restrict__ A, const double *__restrict__ B,
+                                                            const double *__restrict__ LU, double *X,
+                                                            double *__restrict__ rowrms, const int *__restrict__ stop) {
+    extern __shared__ __align__(16) unsigned char gs_smem[];
+    GsShared &S = *reinterpret_cast<GsShared *>(gs_smem);
+    if (stop[0] != 0) return;  // the whole cluster
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int g = lane / 5, m = lane - 5 * g;
+    const bool on = lane < 30;
+    const int q = 6 * w + min(g, 5);          // the group's row in the chunk
+    const int place = blockIdx.x * kGsRows + q;  // and in the cluster's chunk
+    const unsigned group = on ? 31u << (5 * g) : 0u;
+    // the chunk after (level, offset): kGsCtas * kGsRows rows of one level
+    auto advance = [&](int &l, int &at) {
+        at += kGsCtas * kGsRows;
+        while (l < nlevels && at >= ptr[l + 1]) {
+            l++;
+            if (l < nlevels) at = ptr[l];
+        }
+    };
+    auto load_desc = [&](int l, int at) {
+        int4 d = make_int4(-1, 0, 0, 0);
+        if (on && l < nlevels && at + place < ptr[l + 1]) d = desc[at + place];
+        return d;
+    };
+    auto copy = [&](const int4 &d, int buf) {
+        if (d.x >= 0) {
+            GsStage &st = S.stage[buf];
+            const int nb = min(d.z - d.y, kGsBlocks);
+            for (int t = m; t < nb * 25; t += 5) gs_copy8(&st.A[q][t], A + (int64_t)d.y * 25 + t);
+            for (int t = m; t < 25; t += 5) gs_copy8(&st.LU[q][t], LU + (int64_t)d.x * 25 + t);
+            for (int t = m; t < nb; t += 5) gs_copy4(&st.JA[q][t], JA + d.y + t);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    int l = 0, at = ptr[0], ln, an, lf, af;
+    int4 d = load_desc(l, at);
+    copy(d, 0);
+    ln = l; an = at;
+    advance(ln, an);
+    int4 dn = load_desc(ln, an);
+    lf = ln; af = an;
+    if (lf < nlevels) advance(lf, af);
+    double bn = d.x >= 0 ? B[(int64_t)d.x * 5 + m] : 0.0;
+    for (int buf = 0; l < nlevels; buf ^= 1) {
+        copy(dn, buf ^ 1);
+        const int4 df = load_desc(lf, af);
+        const double b0 = bn;
+        bn = dn.x >= 0 ? B[(int64_t)dn.x * 5 + m] : 0.0;
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncwarp();  // a row's copies and reads stay within its warp
+        const GsStage &st = S.stage[buf];
+        if (d.x >= 0) {
+            const int nb = d.z - d.y, ns = min(nb, kGsBlocks);
+            // values of X of the staged blocks: lane m component m
+            double xv[kGsBlocks];
+#pragma unroll
+            for (int t = 0; t < kGsBlocks; t++)
+                xv[t] = t < ns ? __ldcg(X + (int64_t)st.JA[q][t] * 5 + m) : 0.0;
+#pragma unroll
+            for (int t = 0; t < kGsBlocks; t++)
+                if (t < ns) S.x[q][5 * t + m] = xv[t];
+            const double xr = __ldcg(X + (int64_t)d.x * 5 + m);
+            __syncwarp(group);
+            double rhs = b0;
+#pragma unroll 4
+            for (int t = 0; t < ns; t++) {
+                double tv = 0.0;
+#pragma unroll
+                for (int j = 0; j < 5; j++) tv = __dadd_rn(tv, __dmul_rn(st.A[q][t * 25 + m * 5 + j], S.x[q][5 * t + j]));
+                rhs = __dsub_rn(rhs, tv);
+            }
+            for (int k = d.y + kGsBlocks; k < d.z; k++) {
+                const double *a = A + (int64_t)k * 25 + m * 5, *x = X + (int64_t)JA[k] * 5;
+                double tv = 0.0;
+#pragma unroll
+                for (int j = 0; j < 5; j++) tv = __dadd_rn(tv, __dmul_rn(a[j], __ldcg(x + j)));
+                rhs = __dsub_rn(rhs, tv);
+            }
+            double s = 0.0;
+#pragma unroll
+            for (int j = 0; j < 5; j++) {
+                const double v = __shfl_sync(group, rhs, 5 * g + j);
+                s = __dadd_rn(s, __dmul_rn(v, v));
+            }
+            if (m == 0) rowrms[d.x] = s;
+            const int dg = d.w - d.y;
+            double tv = 0.0;
+#pragma unroll
+            for (int j = 0; j < 5; j++) {
+                const double a = dg < kGsBlocks ? st.A[q][dg * 25 + m * 5 + j] : A[(int64_t)d.w * 25 + m * 5 + j];
+                tv = __dadd_rn(tv, __dmul_rn(a, __shfl_sync(group, xr, 5 * g + j)));
+            }
+            rhs = __dadd_rn(rhs, tv);
+            const double *lu = st.LU[q];
+            double v[5], xo[5];
+#pragma unroll
+            for (int ii = 0; ii < 5; ii++) {
+                v[ii] = __shfl_sync(group, rhs, 5 * g + ii);
+#pragma unroll
+                for (int jj = 0; jj < ii; jj++) v[ii] = __dsub_rn(v[ii], __dmul_rn(lu[ii * 5 + jj], v[jj]));
+            }
+            double mine = 0.0;
+#pragma unroll
+            for (int ii = 4; ii >= 0; ii--) {
+                double y = v[ii];
+#pragma unroll
+                for (int jj = 4; jj > ii; jj--) y = __dsub_rn(y, __dmul_rn(lu[ii * 5 + jj], xo[jj]));
+                xo[ii] = __ddiv_rn(y, lu[ii * 5 + ii]);
+                if (m == ii) mine = xo[ii];
+            }
+            X[(int64_t)d.x * 5 + m] = mine;
+        }
+        __syncwarp();
+        // every chunk of a level finishes before the next level starts
+        if (ln != l) {
+            asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+            asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        }
+        l = ln; at = an;
+        d = dn;
+        ln = lf; an = af;
+        dn = df;
+        if (lf < nlevels) advance(lf, af);
+    }
+}
+
+// rms[it] = sqrt(sum / n) of sweep `it`, unless an earlier one stopped; stop
+// {!= 0, sweeps done} (MC_Iterative_Jacobi.c:506)
+__global__ void k_gs_check(const double *__restrict__ sum, int n, int it, double *__restrict__ rms, int *__restrict__ stop) {
+    if (stop[0] != 0) return;
+    const double r = sqrt(sum[0] / (double)n);
+    rms[0] = r;
+    stop[1] = it + 1;
+    if (r < 100.0 * DBL_EPSILON) stop[0] = 1;
+}
+
 // Per-iteration reset: sum(area*lambda) = 0, extrema = (DBL_MAX, DBL_MIN)
 // (Solver_Steady_Implicit.cpp:45-79).
 // Eigenvalue extrema of a residual pass that a limiter fix may supersede:
@@ -1256,6 +1425,7 @@ static Levels *build_levels(const std::vector<int> &IA, const std::vector<int> &
     for (int i = 0; i < n; i++) rows[fill[lev[i]]++] = i;
     L.max_width = 0;
     for (int l = 0; l < nl; l++) L.max_width = std::max(L.max_width, L.ptr[l + 1] - L.ptr[l]);
+    L.desc_built = false;
     err = L.rows.upload(rows.data(), rows.size(), s) == cudaSuccess ? 0 : 1;
     return &L;
 }
@@ -2137,6 +2307,26 @@ int cfd_jacobian(cfd_ctx *c, int add_time, int include_diss, int precision) {
     return CFD_OK;
 }
 
+// Level bounds and row records of k_gs_sweep on the device, once per mesh and direction.
+static int gs_prepare(cfd_ctx *c, int direction) {
+    for (int dir = 0; dir < 2; dir++) {
+        if (direction != 2 && direction != dir) continue;
+        Levels &L = dir == 0 ? c->lv_fwd : c->lv_bwd;
+        if (L.desc_built) continue;
+        std::vector<int> rows(c->nnode);
+        std::vector<int4> desc(c->nnode);
+        CFD_CUDA(cudaMemcpyAsync(rows.data(), L.rows.p, sizeof(int) * c->nnode, cudaMemcpyDeviceToHost, c->stream));
+        CFD_CUDA(stream_wait(c->stream));
+        for (int t = 0; t < c->nnode; t++)
+            desc[t] = make_int4(rows[t], c->h_IA[rows[t]], c->h_IA[rows[t] + 1], c->h_IAU[rows[t]]);
+        CFD_CUDA(L.dptr.upload(L.ptr.data(), L.ptr.size(), c->stream));
+        CFD_CUDA(L.desc.upload(desc.data(), desc.size(), c->stream));
+        CFD_CUDA(stream_wait(c->stream));
+        L.desc_built = true;
+    }
+    return CFD_OK;
+}
+
 int cfd_block_gs(cfd_ctx *c, int iterations, int direction, double *rms) {
     NEED_MESH("cfd_block_gs");
     if (!c->has_system) { set_error("cfd_block_gs: no system (call cfd_jacobian)"); return CFD_ERR_STATE; }
@@ -2154,6 +2344,52 @@ int cfd_block_gs(cfd_ctx *c, int iterations, int direction, double *rms) {
     const int maxit = 10000;
     if (iterations <= 0) iterations = maxit;
     double r = 0.0;
+    // A cluster's sweep while the levels are narrow enough for its eight SMs;
+    // wider ones a launch each.
+    auto narrow = [&](const Levels &L) { return (int64_t)n <= (int64_t)kGsMeanWidth * ((int64_t)L.ptr.size() - 1); };
+    if ((direction == 1 || narrow(c->lv_fwd)) && (direction == 0 || narrow(c->lv_bwd))) {
+        int st = gs_prepare(c, direction);
+        if (st) return st;
+        CFD_CUDA(c->red.alloc(std::max<size_t>(c->red.n, (size_t)296 * 128)));
+        CFD_CUDA(c->red_out.alloc(std::max<size_t>(c->red_out.n, 64)));
+        double *out = c->red_out.p;  // [0] sum, [1] rms, [2] the stop words
+        int *stop = reinterpret_cast<int *>(out + 2);
+        CFD_CUDA(cudaMemsetAsync(out, 0, 4 * sizeof(double), c->stream));
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = kGsCtas;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cudaLaunchConfig_t lc = {};
+        lc.gridDim = dim3(kGsCtas);
+        lc.blockDim = dim3(kGsThreads);
+        lc.dynamicSmemBytes = sizeof(GsShared);
+        lc.stream = c->stream;
+        lc.attrs = at;
+        lc.numAttrs = 1;
+        CFD_CUDA(allow_max_dynamic_smem(k_gs_sweep, c->device, nullptr));
+        struct { double rms; int stop[2]; } back{};
+        // the sweeps' results come back a batch at a time
+        for (int done = 0; done < iterations && !back.stop[0];) {
+            const int last = std::min(iterations, done + 16);
+            for (; done < last; done++) {
+                const bool fwd = direction == 0 || (direction == 2 && done % 2 == 0);
+                const Levels &L = fwd ? c->lv_fwd : c->lv_bwd;
+                CFD_CUDA(cudaLaunchKernelEx(&lc, k_gs_sweep, (int)L.ptr.size() - 1, (const int *)L.dptr.p,
+                                            (const int4 *)L.desc.p, (const int *)c->JA.p, (const double *)c->A64.p,
+                                            (const double *)c->B.p, (const double *)c->LUd.p, c->X.p, c->rowrms.p,
+                                            (const int *)stop));
+                k_sum_partial<<<296, 256, 0, c->stream>>>(c->rowrms.p, n, c->red.p);
+                k_sum_one<<<1, 256, 0, c->stream>>>(c->red.p, 296, out);
+                k_gs_check<<<1, 1, 0, c->stream>>>(out, n, done, out + 1, stop);
+            }
+            CFD_LAUNCH_CHECK();
+            CFD_CUDA(cudaMemcpyAsync(&back, out + 1, sizeof back, cudaMemcpyDeviceToHost, c->stream));
+            CFD_CUDA(stream_wait(c->stream));
+        }
+        r = back.rms;
+        if (rms) *rms = r;
+        return std::isnan(r) ? CFD_ERR_NUMERIC : CFD_OK;
+    }
     for (int it = 0; it < iterations; it++) {
         const bool fwd = direction == 0 || (direction == 2 && it % 2 == 0);
         Levels &L = fwd ? c->lv_fwd : c->lv_bwd;

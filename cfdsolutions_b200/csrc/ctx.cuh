@@ -77,6 +77,9 @@ struct DevBuf {
 struct Levels {
     std::vector<int> ptr;  // host, nlevels+1
     DevBuf<int> rows;      // device, rows in level order
+    bool desc_built = false;  // dptr, desc (k_gs_sweep; built when first used)
+    DevBuf<int> dptr;         // device copy of ptr
+    DevBuf<int4> desc;        // {row, first block, end, diagonal block} in level order
     int max_width = 0;
 };
 
