@@ -278,7 +278,7 @@ __global__ void k_mc_factor(const int *__restrict__ patches, int npatch, int n, 
 
 // Factorisation of the patches of one colour, one CTA of 16 warps per patch:
 // the same operations as the warp-per-patch kernel, for meshes whose patches'
-// blocks fit in shared memory in FP64.  The patch's blocks and lists are
+// blocks fit in shared memory in FP64 (and see kMcWarpPatches).  The patch's blocks and lists are
 // loaded once.  Blocks that couple to other patches come first in every row's
 // order and depend on nothing inside the patch, so the warps, two rows each,
 // eliminate them at once, staging the factor blocks of the other patches.
@@ -293,6 +293,11 @@ __global__ void k_mc_factor(const int *__restrict__ patches, int npatch, int n, 
 constexpr int kMcFactorWarps = 16, kMcFactorRows = kMcRows / kMcFactorWarps;
 static_assert(kMcFactorRows == 2, "two rows per warp");
 constexpr size_t kMcFactorBytes = 222u << 10;  // its shared memory at most
+// FP32 factors of colours with more patches per SM than this go to the warp
+// kernel, whose twenty warps per SM are then all busy: 128^3 cube (41 patches per
+// SM and colour) 22.3 ms per call, 26.1 with a CTA per patch; 96^3 (18) 12.6 and
+// 11.5.  FP64 factors leave it fewer warps: 33.3 and 29.1 ms at 128^3.
+constexpr int kMcWarpPatches = 28;
 __host__ __device__ inline size_t mc_factor_cta_bytes(int maxblk, int maxpairs) {
     return ((size_t)maxblk * (25 * sizeof(double) + sizeof(int4) + 2 * sizeof(int)) + (size_t)maxpairs * sizeof(int2) + 15) &
            ~(size_t)15;
@@ -1171,7 +1176,8 @@ int mc_factor(cfd_ctx *c, const TA *A, TM *M) {
     CFD_CUDA(allow_max_dynamic_smem(k_mc_factor_cta<TA, TM>, c->device, &smax));
     for (int k = 0; k < mc.ncolor; k++) {
         const int cnt = mc.cptr[k + 1] - mc.cptr[k];
-        if (mc.by_cta && smem_cta <= (size_t)smax)
+        const bool many = sizeof(TM) == 4 && cnt > kMcWarpPatches * c->nsm;
+        if (mc.by_cta && smem_cta <= (size_t)smax && !many)
             k_mc_factor_cta<TA, TM><<<cnt, 32 * kMcFactorWarps, smem_cta, c->stream>>>(
                 mc.patches.p + mc.cptr[k], c->nnode, mc.maxblk, mc.maxpairs, mc.stage, c->IA.p, mc.slot.p, mc.meta.p,
                 mc.hdr.p, mc.loc.p, mc.pair_ptr.p, mc.pairs.p, A, M, c->err.p);
