@@ -89,7 +89,7 @@ constexpr int MAXK = 64;
 constexpr int MD_THREADS = 256;
 
 // The block's CH (sum, compensation) pairs of vectors j0 .. j0+nj-1 combined
-// and stored in part[block][j]: a warp butterfly (error-free TwoSum is
+// and stored in part[j][block]: a warp butterfly (error-free TwoSum is
 // symmetric in its arguments, so every lane holds the same pair), then the
 // warps in order.
 template <int CH>
@@ -120,8 +120,7 @@ __device__ __forceinline__ void dot2_block_store(double (&s)[CH], double (&c)[CH
             ss = t;
             cc = (cc + shc[lane][q]) + e;
         }
-        part[(blockIdx.x * MAXK + j0 + lane) * 2] = ss;
-        part[(blockIdx.x * MAXK + j0 + lane) * 2 + 1] = cc;
+        reinterpret_cast<double2 *>(part)[(j0 + lane) * gridDim.x + blockIdx.x] = make_double2(ss, cc);
     }
     __syncthreads();
 }
@@ -234,33 +233,61 @@ __global__ void __launch_bounds__(MD_THREADS) k_axpy_mdot_partial(const double *
     }
 }
 
-__global__ void k_mdot_final(const double *__restrict__ part, int nblk, int k, double *__restrict__ out) {
+// out[j] = the nblk pairs of vector j combined (at most kRedBlocks): a
+// thread's pairs are loaded together, and the last five steps of the tree run
+// in one warp.
+constexpr int kRedBlocks = 1184;  // 8 x 148 SMs
+__global__ void __launch_bounds__(256) k_mdot_final(const double *__restrict__ part, int nblk, double *__restrict__ out) {
     const int j = blockIdx.x;
-    if (j >= k) return;
+    const double2 *p = reinterpret_cast<const double2 *>(part) + (int64_t)j * nblk;
+    constexpr int kPer = (kRedBlocks + 255) / 256;
+    double2 v[kPer];
+#pragma unroll
+    for (int k = 0; k < kPer; k++) {
+        const int b = threadIdx.x + 256 * k;
+        v[k] = b < nblk ? p[b] : make_double2(0.0, 0.0);
+    }
     __shared__ double shs[256], shc[256];
-    double s = 0.0, c = 0.0;
-    for (int b = threadIdx.x; b < nblk; b += blockDim.x) {
+    double s = v[0].x, c = v[0].y;
+#pragma unroll
+    for (int k = 1; k < kPer; k++) {
         double t, e;
-        two_sum(s, part[(b * MAXK + j) * 2], t, e);
+        two_sum(s, v[k].x, t, e);
         s = t;
-        c += e + part[(b * MAXK + j) * 2 + 1];
+        c += e + v[k].y;
     }
     shs[threadIdx.x] = s;
     shc[threadIdx.x] = c;
     __syncthreads();
-    for (int o = blockDim.x >> 1; o > 0; o >>= 1) {
+    for (int o = 128; o >= 32; o >>= 1) {
         if (threadIdx.x < o) {
             double t, e;
-            two_sum(shs[threadIdx.x], shs[threadIdx.x + o], t, e);
-            shs[threadIdx.x] = t;
-            shc[threadIdx.x] += shc[threadIdx.x + o] + e;
+            two_sum(s, shs[threadIdx.x + o], t, e);
+            s = t;
+            c += shc[threadIdx.x + o] + e;
+            shs[threadIdx.x] = s;
+            shc[threadIdx.x] = c;
         }
         __syncthreads();
     }
-    if (threadIdx.x == 0) out[j] = shs[0] + shc[0];
+    if (threadIdx.x >= 32) return;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const double so = __shfl_down_sync(0xffffffffu, s, o), co = __shfl_down_sync(0xffffffffu, c, o);
+        double t, e;
+        two_sum(s, so, t, e);
+        s = t;
+        c += co + e;
+    }
+    if (threadIdx.x == 0) out[j] = s + c;
 }
 
-static const int kRedBlocks = 1184;  // 8 x 148 SMs
+// Blocks of the Dot2 reductions over n elements: four elements per thread
+// before a second wave of blocks pays; the grid fixes the order of the sums,
+// so it depends on n alone.
+static int red_blocks(int64_t n) {
+    return (int)std::min<int64_t>(kRedBlocks, std::max<int64_t>(148, n / (4 * MD_THREADS)));
+}
 
 // Device scalars of the GMRES driver, in c->dots (doubles):
 //   [0, MAXK)        dot results read back by the host; [MAXK/2, MAXK) also
@@ -275,11 +302,12 @@ constexpr int DOT_H1 = MAXK, DOT_H2 = 2 * MAXK, DOT_COL = 3 * MAXK, DOT_NRM = 4 
 // The chunk width follows k and the elements per step shrink as it grows, to
 // keep the registers (and so the resident blocks) and the loads in flight up.
 static int mdot_dev(cfd_ctx *c, const double *V, int64_t ld, int k, const double *w, int64_t n, double *out_dev) {
-    if (k <= 1) k_mdot_partial<1, 8><<<kRedBlocks, MD_THREADS, 0, c->stream>>>(V, ld, k, w, n, c->red.p);
-    else if (k <= 4) k_mdot_partial<4, 4><<<kRedBlocks, MD_THREADS, 0, c->stream>>>(V, ld, k, w, n, c->red.p);
-    else k_mdot_partial<8, 2><<<kRedBlocks, MD_THREADS, 0, c->stream>>>(V, ld, k, w, n, c->red.p);
+    const int g = red_blocks(n);
+    if (k <= 1) k_mdot_partial<1, 8><<<g, MD_THREADS, 0, c->stream>>>(V, ld, k, w, n, c->red.p);
+    else if (k <= 4) k_mdot_partial<4, 4><<<g, MD_THREADS, 0, c->stream>>>(V, ld, k, w, n, c->red.p);
+    else k_mdot_partial<8, 2><<<g, MD_THREADS, 0, c->stream>>>(V, ld, k, w, n, c->red.p);
     CFD_LAUNCH_CHECK();
-    k_mdot_final<<<k, 256, 0, c->stream>>>(c->red.p, kRedBlocks, k, out_dev);
+    k_mdot_final<<<k, 256, 0, c->stream>>>(c->red.p, g, out_dev);
     CFD_LAUNCH_CHECK();
     return CFD_OK;
 }
@@ -288,14 +316,14 @@ static int mdot_dev(cfd_ctx *c, const double *V, int64_t ld, int k, const double
 // (j < k) or, self, out_dev[0] = <w, w>: the update and mdot_dev in one pass.
 static int axpy_mdot_dev(cfd_ctx *c, const double *V, int64_t ld, int k, const double *h_dev, double *w, int64_t n,
                          bool self, double *out_dev) {
-    const int g = kRedBlocks, t = MD_THREADS;
+    const int g = red_blocks(n), t = MD_THREADS;
     double *part = c->red.p;
     if (self) k_axpy_mdot_partial<true, 1, 4><<<g, t, 0, c->stream>>>(V, ld, k, h_dev, w, n, part);
     else if (k <= 4) k_axpy_mdot_partial<false, 4, 4><<<g, t, 0, c->stream>>>(V, ld, k, h_dev, w, n, part);
     else k_axpy_mdot_partial<false, 8, 2><<<g, t, 0, c->stream>>>(V, ld, k, h_dev, w, n, part);
     CFD_LAUNCH_CHECK();
     const int kd = self ? 1 : k;
-    k_mdot_final<<<kd, 256, 0, c->stream>>>(c->red.p, kRedBlocks, kd, out_dev);
+    k_mdot_final<<<kd, 256, 0, c->stream>>>(c->red.p, g, out_dev);
     CFD_LAUNCH_CHECK();
     return CFD_OK;
 }
