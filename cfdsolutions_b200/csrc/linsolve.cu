@@ -841,9 +841,10 @@ static int vnorm(cfd_ctx *c, const double *x, int64_t n, double *out) {
 // Restarted right-preconditioned GMRES(m) for A_p d = r (A_p = A in storage
 // precision `aprec`), d starting at zero.  Classical Gram-Schmidt with one
 // re-orthogonalisation pass (CGS2), compensated FP64 dot products, Givens
-// rotations on the host.  Returns inner iterations in *its.
+// rotations on the host.  rn = ||r||.  Returns inner iterations in *its and
+// ||r - A_p d||, evaluated anew after every restart, in *res_est.
 static int gmres_inner(cfd_ctx *c, int aprec, const Precond &pc, int m, int max_iters, double tol_abs,
-                       const double *r, double *d, int *its, int *restarts, double *res_est) {
+                       const double *r, double rn, double *d, int *its, int *restarts, double *res_est) {
     const int64_t n5 = (int64_t)c->nnode * 5;
     const int64_t ld = n5;
     double *V = c->V.p;
@@ -854,15 +855,12 @@ static int gmres_inner(cfd_ctx *c, int aprec, const Precond &pc, int m, int max_
     int st0 = dot_buffers(c);
     if (st0) return st0;
     CFD_CUDA(cudaMemsetAsync(d, 0, n5 * sizeof(double), c->stream));
-    CFD_CUDA(cudaMemcpyAsync(w, r, n5 * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
-    int total = 0, nrst = 0;
-    double beta;
-    int st = vnorm(c, w, n5, &beta);
-    if (st) return st;
+    int total = 0, nrst = 0, st = CFD_OK;
+    double beta = rn;
     *res_est = beta;
     while (total < max_iters && beta > tol_abs) {
         if (!std::isfinite(beta)) { set_error("gmres: non-finite residual"); return CFD_ERR_NUMERIC; }
-        k_scale_copy<<<1184, 256, 0, c->stream>>>(n5, 1.0 / beta, w, V);
+        k_scale_copy<<<1184, 256, 0, c->stream>>>(n5, 1.0 / beta, nrst == 0 ? r : w, V);
         std::fill(g.begin(), g.end(), 0.0);
         g[0] = beta;
         int j = 0;
@@ -1026,37 +1024,51 @@ int cfd_gmres(cfd_ctx *c, const cfd_gmres_opts *o, cfd_gmres_stats *stats) {
         return CFD_OK;
     }
     const int nref = std::max(1, opt.refine);
-    double rel = 1.0;
+    // the matrix that the FP64 defects use (spmv(c, CFD_PREC_FP64, ..)) is the one inside GMRES
+    const bool same_matrix = !c->a64_valid || aprec == CFD_PREC_FP64;
+    double rel = 1.0, rn = bnorm;
+    bool known = true;  // rn is ||B - A x||
     int left = opt.max_iters;
     for (int it = 0; it < nref && left > 0; it++) {
-        // FP64 defect: r = B - A64 x
-        if ((st = spmv(c, CFD_PREC_FP64, x, r))) return st;
-        k_sub<<<1184, 256, 0, c->stream>>>(n5, c->B.p, r, r);
-        CFD_LAUNCH_CHECK();
-        double rn;
-        if ((st = vnorm(c, r, n5, &rn))) return st;
+        // FP64 defect: r = B - A64 x, which is B in the first sweep (x = 0)
+        if (it > 0) {
+            if ((st = spmv(c, CFD_PREC_FP64, x, r))) return st;
+            k_sub<<<1184, 256, 0, c->stream>>>(n5, c->B.p, r, r);
+            CFD_LAUNCH_CHECK();
+            if ((st = vnorm(c, r, n5, &rn))) return st;
+            known = true;
+        }
         rel = rn / bnorm;
         if (rel <= opt.rtol) break;
         int its = 0, rs = 0;
         double est = 0.0;
         // inner tolerance relative to this defect; the final check is FP64
         const double tol_abs = std::max(opt.rtol * bnorm, (nref > 1 ? 1e-3 : 1.0) * opt.rtol * rn);
-        st = gmres_inner(c, aprec, pc, m, left, nref > 1 ? std::max(opt.rtol * bnorm, 1e-4 * rn) : tol_abs, r, d,
-                         &its, &rs, &est);
-        if (st) return st;
-        k_add<<<1184, 256, 0, c->stream>>>(n5, d, x);
-        CFD_LAUNCH_CHECK();
+        st = gmres_inner(c, aprec, pc, m, left, nref > 1 ? std::max(opt.rtol * bnorm, 1e-4 * rn) : tol_abs,
+                         it > 0 ? r : c->B.p, rn, it > 0 ? d : x, &its, &rs, &est);
+        if (st) {
+            if (it == 0) CFD_CUDA(cudaMemsetAsync(x, 0, n5 * sizeof(double), c->stream));  // no partial solution
+            return st;
+        }
+        if (it > 0) {
+            k_add<<<1184, 256, 0, c->stream>>>(n5, d, x);
+            CFD_LAUNCH_CHECK();
+        }
+        // the first sweep's own residual is the defect of x: nothing to evaluate again
+        known = it == 0 && same_matrix;
+        rn = est;
         s.iterations += its;
         s.restarts += rs;
         s.refinements = it + 1;
         left -= its;
     }
     // final FP64 residual
-    if ((st = spmv(c, CFD_PREC_FP64, x, r))) return st;
-    k_sub<<<1184, 256, 0, c->stream>>>(n5, c->B.p, r, r);
-    CFD_LAUNCH_CHECK();
-    double rn;
-    if ((st = vnorm(c, r, n5, &rn))) return st;
+    if (!known) {
+        if ((st = spmv(c, CFD_PREC_FP64, x, r))) return st;
+        k_sub<<<1184, 256, 0, c->stream>>>(n5, c->B.p, r, r);
+        CFD_LAUNCH_CHECK();
+        if ((st = vnorm(c, r, n5, &rn))) return st;
+    }
     s.rel_residual = rn / bnorm;
     if (stats) *stats = s;
     if (!std::isfinite(s.rel_residual)) {
