@@ -805,11 +805,16 @@ int mc_build(cfd_ctx *c) {
     const int n = c->nnode;
     const std::vector<int> &IA = c->h_IA, &JA = c->h_JA, &IAU = c->h_IAU;
     const int np = (n + kMcRows - 1) / kMcRows;
-    // ranges of patches, on as many threads as their rows are worth (a row's
-    // share of a patch's loops outweighs an item of the plain ones)
+    // ranges of patches or rows, on as many threads as their rows are worth (a
+    // row's lists cost some microseconds, an item of a plain loop nanoseconds)
+    constexpr int kRowWeight = 16;
     auto parallel_patches = [&](auto fn) {
-        const int64_t items = 4 * (int64_t)n;
+        const int64_t items = kRowWeight * (int64_t)n;
         parallel_ranges(items, [&](int t, int64_t i0, int64_t i1) { fn(t, i0 * np / items, i1 * np / items); });
+    };
+    auto parallel_rows = [&](auto fn) {
+        const int64_t items = kRowWeight * (int64_t)n;
+        parallel_ranges(items, [&](int, int64_t i0, int64_t i1) { fn((int)(i0 / kRowWeight), (int)(i1 / kRowWeight)); });
     };
     // DSATUR colouring of the patch graph (Brelaz 1979): repeatedly colour the
     // uncoloured patch with the most distinct colours among its neighbours
@@ -1103,8 +1108,8 @@ int mc_build(cfd_ctx *c) {
         if (out) ext_pairs[i] = next_pairs;
         return total;
     };
-    parallel_ranges(n, [&](int, int64_t i0, int64_t i1) {
-        for (int i = (int)i0; i < (int)i1; i++) pair_ptr[i + 1] = row_pairs(i, nullptr);
+    parallel_rows([&](int i0, int i1) {
+        for (int i = i0; i < i1; i++) pair_ptr[i + 1] = row_pairs(i, nullptr);
     });
     int maxstage = 1;
     for (int i = 0; i < n; i++) {
@@ -1115,8 +1120,8 @@ int mc_build(cfd_ctx *c) {
     for (int P = 0; P < np; P++)
         maxpairs = std::max(maxpairs, pair_ptr[std::min(n, (P + 1) * kMcRows)] - pair_ptr[P * kMcRows]);
     std::vector<int2> pairs(std::max<int64_t>(pair_ptr[n], 1));
-    parallel_ranges(n, [&](int, int64_t i0, int64_t i1) {
-        for (int i = (int)i0; i < (int)i1; i++) row_pairs(i, pairs.data() + pair_ptr[i]);
+    parallel_rows([&](int i0, int i1) {
+        for (int i = i0; i < i1; i++) row_pairs(i, pairs.data() + pair_ptr[i]);
     });
     int maxcnt = 0;
     for (int i = 0; i < n; i++) {
