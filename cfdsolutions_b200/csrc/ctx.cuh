@@ -108,9 +108,12 @@ struct Abmc {
     DevBuf<int4> desc[2];
     DevBuf<uint4> lists[2];
     std::vector<int4> shape[2];
-    // captured applies (one CUDA graph per factor / input / scratch / output
-    // pointer set; the GMRES driver reuses a few such sets)
+    // captured applies (one CUDA graph per factor type and factor / input /
+    // scratch / output pointer set; the GMRES driver reuses a few such sets).
+    // The factors are replaced whenever another preconditioner needs a buffer
+    // of another size, so FP32 factors may lie where FP64 ones lay.
     struct Graph {
+        size_t elem;  // bytes per element of M
         const void *M, *r, *tmp, *z;
         cudaGraphExec_t exec;
     };

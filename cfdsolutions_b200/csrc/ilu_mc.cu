@@ -1241,13 +1241,13 @@ static int mc_apply_launch(cfd_ctx *c, const TM *M, const double *r, double *tmp
 // The 2 x ncolor launches of an apply, replayed as one captured CUDA graph
 // when the context has its own stream (the legacy stream cannot be
 // captured): the host then issues one launch instead of 2 x ncolor, which is
-// what bounds small systems.  Graphs are cached per pointer set.
+// what bounds small systems.  Graphs are cached per factor type and pointer set.
 template <typename TM>
 int mc_apply(cfd_ctx *c, const TM *M, const double *r, double *tmp, double *z) {
     Abmc &mc = c->mc;
     if (!c->stream) return mc_apply_launch<TM>(c, M, r, tmp, z);
     for (const auto &g : mc.graphs)
-        if (g.M == M && g.r == r && g.tmp == tmp && g.z == z) {
+        if (g.elem == sizeof(TM) && g.M == M && g.r == r && g.tmp == tmp && g.z == z) {
             CFD_CUDA(cudaGraphLaunch(g.exec, c->stream));
             return CFD_OK;
         }
@@ -1265,7 +1265,7 @@ int mc_apply(cfd_ctx *c, const TM *M, const double *r, double *tmp, double *z) {
     const cudaError_t ei = cudaGraphInstantiate(&exec, graph, 0);
     cudaGraphDestroy(graph);
     CFD_CUDA(ei);
-    mc.graphs.push_back({M, r, tmp, z, exec});
+    mc.graphs.push_back({sizeof(TM), M, r, tmp, z, exec});
     CFD_CUDA(cudaGraphLaunch(exec, c->stream));
     return CFD_OK;
 }
