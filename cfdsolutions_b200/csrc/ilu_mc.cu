@@ -491,7 +491,7 @@ __device__ __forceinline__ void copy16(void *smem, const void *gmem) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem)
                  : "memory");
 }
-// Starts fetching [gmem, gmem + bytes) from DRAM into L2 (multiples of 16).
+// Starts fetching [gmem, gmem + bytes) from DRAM into L2 (bytes > 0, multiples of 16).
 __device__ __forceinline__ void prefetch_l2(const void *gmem, unsigned bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(gmem), "r"(bytes) : "memory");
 }
@@ -601,7 +601,8 @@ __global__ void __launch_bounds__(kMcSolveThreads, 5) k_mc_solve(const int4 *__r
         // a patch that a later wave of this grid takes
         if (tid == 0 && blockIdx.x + kMcAheadPatches < gridDim.x) {
             const int4 f = desc[blockIdx.x + kMcAheadPatches];
-            prefetch_l2(M + (int64_t)f.z * kMcUnit, (unsigned)(f.w * kMcUnit * sizeof(TM)));
+            // a patch without lower blocks has an empty region, which may begin at the end of M
+            if (f.w > 0) prefetch_l2(M + (int64_t)f.z * kMcUnit, (unsigned)(f.w * kMcUnit * sizeof(TM)));
             prefetch_l2(lists + f.x, (unsigned)f.y * 16u);
         }
         copy_wait();
