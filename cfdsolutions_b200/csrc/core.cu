@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cfloat>
 #include <cmath>
 #include <cstdarg>
@@ -674,7 +675,7 @@ __global__ void __launch_bounds__(32 * JAC_WARPS, MODE == 1 ? 2 : 3) k_jacobian(
     if (i - lane >= nnode) return;  // whole warps past the end
     const bool live = i < nnode;
     const int row = live ? i : nnode - 1;
-    const int d = live ? deg[row] : 0, first = IA[row], end = IA[row + 1];
+    const int d = live ? deg[row] : 0, first = IA[row];
     const int64_t base = sell_ptr[row >> 5] + lane;
     const int steps = (int)((sell_ptr[(row >> 5) + 1] - sell_ptr[row >> 5]) / 32);
     double qi[5], D[25];
@@ -749,9 +750,9 @@ __global__ void __launch_bounds__(32 * JAC_WARPS, MODE == 1 ? 2 : 3) k_jacobian(
                 const double other = ha * (-sg * J[m] - Ab[m]);
                 D[m] -= HIGH ? other : round_low<TA>(other);
             }
-            // block k of the row, the diagonal one lying before those of larger columns
+            // block k of the row, the diagonal one lying before those of larger
+            // columns (the block pattern is that of the edges: require_edge_graph)
             slot = first + k + (j > row ? 1 : 0);
-            if (slot >= end) slot = -1;
         }
         store(slot);
     }
@@ -1134,6 +1135,12 @@ int check_device_error(cfd_ctx *c) {
         return CFD_ERR_NUMERIC;
     }
     return CFD_OK;
+}
+
+int require_edge_graph(cfd_ctx *c, const char *who) {
+    if (c->graph_is_edges) return CFD_OK;
+    set_error("%s: the rows of the mesh's node graph (n2n) are not the neighbours that its edges give", who);
+    return CFD_ERR_MESH;
 }
 
 // Far-field state with Mach ramping (ComputeFarFieldCondition,
@@ -2004,6 +2011,7 @@ int cfd_set_mesh(cfd_ctx *c, int nnode, int nghost, int nedge, const int *edge_n
             nb[fill[a]] = b; lst[fill[a]++] = e;
             nb[fill[b]] = a; lst[fill[b]++] = ~e;
         }
+        std::atomic<bool> same{true};
         parallel_ranges(nnode, [&](int, int64_t r0, int64_t r1) {
             std::vector<int> idx, tmp;
             for (int64_t i = r0; i < r1; i++) {
@@ -2014,8 +2022,13 @@ int cfd_set_mesh(cfd_ctx *c, int nnode, int nghost, int nedge, const int *edge_n
                 tmp.resize(hi - lo);
                 for (int k = 0; k < hi - lo; k++) tmp[k] = lst[idx[k]];
                 std::copy(tmp.begin(), tmp.end(), lst.begin() + lo);
+                bool ok = hi - lo == gia[i + 1] - gia[i];
+                for (int k = 0; ok && k < hi - lo; k++)
+                    ok = nb[idx[k]] == gja[gia[i] + k] && (k == 0 || nb[idx[k]] > nb[idx[k - 1]]);
+                if (!ok) same = false;
             }
         });
+        c->graph_is_edges = same;
         CFD_CUDA(c->n2e_ptr.upload(ptr.data(), ptr.size(), s));
         CFD_CUDA(c->n2e.upload(lst.data(), lst.size(), s));
         CFD_CUDA(stream_wait(s));
@@ -2288,6 +2301,8 @@ int cfd_jacobian(cfd_ctx *c, int add_time, int include_diss, int precision) {
         set_error("cfd_jacobian: precision must be FP64, FP32 or BF16 (LOW_ONLY with FP32/BF16)");
         return CFD_ERR_ARG;
     }
+    int st = require_edge_graph(c, "cfd_jacobian");
+    if (st) return st;
     if (!low_only) CFD_CUDA(c->A64.alloc((size_t)c->nnzb * 25));
     CFD_CUDA(c->B.alloc((size_t)c->nnode * 5));
     CFD_CUDA(c->X.alloc((size_t)c->nnode * 5));

@@ -225,6 +225,7 @@ struct cfd_ctx {
     cfd::Flow flow{};
     double cfl = 0.0;
     bool has_mesh = false;
+    bool graph_is_edges = false;  // every row of the node graph holds its edges' other nodes, each once
 
     int nnode = 0, nghost = 0, nedge = 0, nbedge = 0;
     int64_t nnzb = 0;
@@ -377,6 +378,9 @@ enum : int {
 };
 
 int check_device_error(cfd_ctx *c);
+// CFD_ERR_MESH unless the node graph is that of the edges (the Jacobians then
+// know every edge's blocks by their place).
+int require_edge_graph(cfd_ctx *c, const char *who);
 // fused Green-Gauss + limiter pass over nodes [lo, hi) (gradient.cu), limiters
 // to phi_out, the reconstructed-pressure check left to the residual
 int gg_limiter_range(cfd_ctx *c, double *phi_out, int lo, int hi);

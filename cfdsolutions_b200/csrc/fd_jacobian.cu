@@ -405,6 +405,8 @@ extern "C" int cfd_jacobian_fd(cfd_ctx *c, int add_time, int include_diss, int m
                   "without the low-Mach fix)");
         return CFD_ERR_UNSUPPORTED;
     }
+    int st = require_edge_graph(c, "cfd_jacobian_fd");
+    if (st) return st;
     CFD_CUDA(cudaSetDevice(c->device));
     if (method == CFD_JAC_ALTERNATE)  // Roe_Jacobian.cpp:282-287
         method = iteration % 2 == 0 ? CFD_JAC_FORWARD : CFD_JAC_BACKWARD;

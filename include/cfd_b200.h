@@ -203,7 +203,9 @@ int  cfd_synchronize(cfd_ctx *ctx);
  *   edge_nodes  [2*nedge]   edge_areav  [3*nedge]
  *   bedge_nodes [2*nbedge]  bedge_areav [3*nbedge]  bedge_type [nbedge]
  *   cvol [nnode]  coords [3*nnode] (xyz interleaved, as coordXYZ)
- *   n2n_ia [nnode+1]  n2n_ja [n2n_ia[nnode]]  (no diagonal) */
+ *   n2n_ia [nnode+1]  n2n_ja [n2n_ia[nnode]]  (no diagonal)
+ * The Jacobians need rows of n2n that hold the other nodes of the row's edges,
+ * each once, and return CFD_ERR_MESH otherwise. */
 int  cfd_set_mesh(cfd_ctx *ctx, int nnode, int nghost,
                   int nedge, const int *edge_nodes, const double *edge_areav,
                   int nbedge, const int *bedge_nodes, const double *bedge_areav,
