@@ -348,7 +348,7 @@ __global__ void k_arnoldi_column(int j, double *__restrict__ dots) {
     const int i = threadIdx.x;
     if (i <= j) dots[DOT_COL + i] = dots[DOT_H1 + i] + dots[DOT_H2 + i];
     if (i == 0) {
-        const double hn = sqrt(fmax(dots[DOT_NRM], 0.0));
+        const double nn = dots[DOT_NRM], hn = sqrt(nn < 0.0 ? 0.0 : nn);  // a NaN stays one
         dots[DOT_COL + j + 1] = hn;
         dots[DOT_COL + MAXK - 1] = hn > 0.0 ? 1.0 / hn : 0.0;
     }
@@ -834,7 +834,7 @@ static int vnorm(cfd_ctx *c, const double *x, int64_t n, double *out) {
     double s;
     int st = mdot(c, x, 0, 1, x, n, &s);
     if (st) return st;
-    *out = sqrt(fmax(s, 0.0));
+    *out = sqrt(s < 0.0 ? 0.0 : s);  // a NaN stays one
     return CFD_OK;
 }
 
@@ -1027,7 +1027,7 @@ int cfd_gmres(cfd_ctx *c, const cfd_gmres_opts *o, cfd_gmres_stats *stats) {
     // the matrix that the FP64 defects use (spmv(c, CFD_PREC_FP64, ..)) is the one inside GMRES
     const bool same_matrix = !c->a64_valid || aprec == CFD_PREC_FP64;
     double rel = 1.0, rn = bnorm;
-    bool known = true;  // rn is ||B - A x||
+    bool known = false;  // rn is ||B - A x||, evaluated
     int left = opt.max_iters;
     for (int it = 0; it < nref && left > 0; it++) {
         // FP64 defect: r = B - A64 x, which is B in the first sweep (x = 0)
