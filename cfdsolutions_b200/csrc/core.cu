@@ -2363,9 +2363,29 @@ int cfd_block_gs(cfd_ctx *c, int iterations, int direction, double *rms) {
     if (iterations <= 0) iterations = maxit;
     double r = 0.0;
     // A cluster's sweep while the levels are narrow enough for its eight SMs;
-    // wider ones a launch each.
+    // wider ones a launch each, and all of them where no such cluster can be
+    // resident (a partitioned GPU).
     auto narrow = [&](const Levels &L) { return (int64_t)n <= (int64_t)kGsMeanWidth * ((int64_t)L.ptr.size() - 1); };
-    if ((direction == 1 || narrow(c->lv_fwd)) && (direction == 0 || narrow(c->lv_bwd))) {
+    bool cluster = (direction == 1 || narrow(c->lv_fwd)) && (direction == 0 || narrow(c->lv_bwd));
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = kGsCtas;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3(kGsCtas);
+    lc.blockDim = dim3(kGsThreads);
+    lc.dynamicSmemBytes = sizeof(GsShared);
+    lc.stream = c->stream;
+    lc.attrs = at;
+    lc.numAttrs = 1;
+    if (cluster) {
+        int smax = 0, resident = 0;
+        CFD_CUDA(allow_max_dynamic_smem(k_gs_sweep, c->device, &smax));
+        cluster = sizeof(GsShared) <= (size_t)smax &&
+                  cudaOccupancyMaxActiveClusters(&resident, k_gs_sweep, &lc) == cudaSuccess && resident > 0;
+        if (!cluster) (void)cudaGetLastError();
+    }
+    if (cluster) {
         int st = gs_prepare(c, direction);
         if (st) return st;
         CFD_CUDA(c->red.alloc(std::max<size_t>(c->red.n, (size_t)296 * 128)));
@@ -2373,18 +2393,6 @@ int cfd_block_gs(cfd_ctx *c, int iterations, int direction, double *rms) {
         double *out = c->red_out.p;  // [0] sum, [1] rms, [2] the stop words
         int *stop = reinterpret_cast<int *>(out + 2);
         CFD_CUDA(cudaMemsetAsync(out, 0, 4 * sizeof(double), c->stream));
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = kGsCtas;
-        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-        cudaLaunchConfig_t lc = {};
-        lc.gridDim = dim3(kGsCtas);
-        lc.blockDim = dim3(kGsThreads);
-        lc.dynamicSmemBytes = sizeof(GsShared);
-        lc.stream = c->stream;
-        lc.attrs = at;
-        lc.numAttrs = 1;
-        CFD_CUDA(allow_max_dynamic_smem(k_gs_sweep, c->device, nullptr));
         struct { double rms; int stop[2]; } back{};
         // the sweeps' results come back a batch at a time
         for (int done = 0; done < iterations && !back.stop[0];) {
