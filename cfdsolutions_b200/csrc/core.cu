@@ -895,18 +895,26 @@ __global__ void __launch_bounds__(128) k_gs_level(int nrows, const int *__restri
 }
 
 // A whole sweep in one launch: one cluster of kGsCtas CTAs walks the levels,
-// separated by the cluster's hardware barrier, where a launch per level cost
-// 19 us for some hundred rows.  Five lanes per row (six rows per warp), lane m
+// separated by the cluster's hardware barrier, where a launch per level costs
+// 28 us for some hundred rows.  Five lanes per row (six rows per warp), lane m
 // forming component m with k_gs_level's operations in the same order.  What
 // does not depend on X -- a row's blocks, its LU factors and column ids -- is
 // copied to shared memory one chunk of rows ahead, across level bounds; after
 // the barrier one round trip to L2 fetches the values of X.
 constexpr int kGsCtas = 8, kGsWarps = 4, kGsRows = 6 * kGsWarps, kGsThreads = 32 * kGsWarps;
 constexpr int kGsBlocks = 16;  // blocks of a row staged (the rest are read from global memory)
-// Mean rows per level up to which the cluster sweeps.  Ten sweeps, launches per
-// level / cluster: 20^3 cube (120 rows per level) 19.8 / 5.1 ms, 40^3 147 / 32,
-// 64^3 265 / 103, 96^3 (1300) 396 / 312.
-constexpr int kGsMeanWidth = 2048;
+// Mean rows per level up to which the cluster sweeps.  The cluster pays by the
+// row, 23 / 34 / 83 ns for rows of 7 / 15 / 40 blocks, the launches by the level,
+// 31 / 51-62 / 167 us (no more for 1800 rows than for 800: latency).  They break
+// even near 1350 rows (hexahedra; sweep of the 80^3 box, 1262 rows per level:
+// launches 13.5 ms, cluster 12.6; 88^3, 1516: 15.0 and 16.5) and between 1500
+// and 1800 (tets: 64^3 in natural order, 1423: 9.8 and 9.2; blocked RCM 96^3,
+// 1383: 39.7 and 31.2; 112^3, 1764: 49.5 and 48.3; 120^3, 2060: 52.0 and 58.9);
+// with 40 blocks 1750 rows still gain (8.4 and 7.3 ms).  20^3 (116 rows): 2.0 and
+// 0.51 ms.
+static bool gs_narrow(int64_t n, int64_t nnzb, int64_t levels) {
+    return n <= levels * std::min<int64_t>(1750, 1000 + 35 * nnzb / n);
+}
 struct GsStage {
     double A[kGsRows][kGsBlocks * 25];
     double LU[kGsRows][25];
@@ -2365,7 +2373,7 @@ int cfd_block_gs(cfd_ctx *c, int iterations, int direction, double *rms) {
     // A cluster's sweep while the levels are narrow enough for its eight SMs;
     // wider ones a launch each, and all of them where no such cluster can be
     // resident (a partitioned GPU).
-    auto narrow = [&](const Levels &L) { return (int64_t)n <= (int64_t)kGsMeanWidth * ((int64_t)L.ptr.size() - 1); };
+    auto narrow = [&](const Levels &L) { return gs_narrow(n, c->nnzb, (int64_t)L.ptr.size() - 1); };
     bool cluster = (direction == 1 || narrow(c->lv_fwd)) && (direction == 0 || narrow(c->lv_bwd));
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
