@@ -634,23 +634,33 @@ __global__ void k_add_diss(int64_t n, const double *__restrict__ a, const double
 // sides:
 //   A[i,i] = V_i/dt_i I - sum_j A[j,i] + sum_b 0.5 (J(Q_i) + |A|)_b area_b
 //   B_i    = -(Res_i [+ Res_Diss_i])
-// One thread per row walks its edges (the sliced-ELL incidence, whose order is
-// that of the row's blocks) and forms both blocks of each: its own, stored,
-// and the transposed one, added to its diagonal block in registers.  Every edge
-// is evaluated from both ends, in the same orientation and so to the same bits,
-// and no block is read back: the two passes this replaces (edges, then rows
-// that gathered the transposed blocks) moved the blocks three times, half of
-// it in partial sectors.  Measured on the 96^3 cube, FP32 / FP64 blocks: 1067 /
-// 1268 us (before: 1430 / 1632), 24^3 43 / 41 us (58 / 61).  Bound by the FP64
-// pipe and by latency at three CTAs per SM (168 registers).  The lanes stage their blocks in
-// shared memory and the warp stores them one after the other, 100 or 200
-// contiguous bytes each; a row's next block follows in the next step, so the
-// sectors they share fill in L2.
+// LANES threads per row (see kJacLanesRows) walk its edges (the sliced-ELL
+// incidence, whose order is that of the row's blocks) and form both blocks of
+// each: its own, stored, and the transposed one, added to the diagonal block in
+// registers.  Every edge is evaluated from both ends, in the same orientation
+// and so to the same bits, and no block is read back: the two passes this
+// replaces (edges, then rows that gathered the transposed blocks) moved the
+// blocks three times, half of it in partial sectors.  Measured on the 96^3
+// cube, FP32 / FP64 blocks: 1067 / 1268 us (before: 1430 / 1632), 24^3 34 / 33
+// us (58 / 61).  Bound by latency at three CTAs per SM (168 registers).  The
+// lanes stage their blocks in shared memory and the warp stores them one after
+// the other, 100 or 200 contiguous bytes each; a row's next block follows in
+// the next step, so the sectors they share fill in L2.
 // The low-precision-only system sums the diagonal from the rounded blocks.
 // MODE: 0 Roe, 1 preconditioned Roe (CFD_FLUX_ROE_PRECOND), 2 Thornber (|A| of
 // the modified states).  RUP: the state's variables (f.rup).  HIGH / LOW: an
 // FP64 / a low-precision matrix is stored.
 constexpr int JAC_WARPS = 4;  // warps per CTA
+// Rows up to which four lanes share a row, every fourth edge each, and add their
+// parts of the diagonal block at the end.  A thread per row leaves most SMs'
+// warp slots empty up to 148 SMs x 12 warps x 32 lanes / 4, and each thread then
+// works off its edges one behind the other: 8^3 cube (729 rows), Roe FP64 39.5 /
+// 14.9 us with 1 / 4 lanes, preconditioned Roe 78.9 / 29.2, 24^3 (15,625 rows)
+// 41.4 / 33.2 and 80.4 / 64.2; 64^3 FP32 347 / 377, preconditioned 724 / 865.
+// With two matrices stored, FP64 and a low-precision one, four lanes are the
+// faster at every size but small boxes of hexahedra (tets 24^3 70 / 49 us, 48^3
+// 346 / 269, 80^3 1300 / 1128; hexahedra 32^3 41 / 48, 64^3 324 / 332).
+constexpr int kJacLanesRows = 16000;
 
 template <typename TA>
 __device__ __forceinline__ double round_low(double v) {
@@ -659,7 +669,7 @@ __device__ __forceinline__ double round_low(double v) {
     return load_low(&t);
 }
 
-template <typename TA, int MODE, bool RUP, bool HIGH, bool LOW>
+template <typename TA, int MODE, bool RUP, bool HIGH, bool LOW, int LANES>
 __global__ void __launch_bounds__(32 * JAC_WARPS, MODE == 1 ? 2 : 3) k_jacobian(
     int nnode, int64_t ldq, const double *__restrict__ Q, const int *__restrict__ IA, const int *__restrict__ IAU,
     const int64_t *__restrict__ sell_ptr, const int *__restrict__ sell_nbr, const double4 *__restrict__ sell_geo,
@@ -671,12 +681,12 @@ __global__ void __launch_bounds__(32 * JAC_WARPS, MODE == 1 ? 2 : 3) k_jacobian(
     using TS = std::conditional_t<HIGH, double, TA>;  // staged blocks
     __shared__ TS stage[JAC_WARPS][32][25];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i - lane >= nnode) return;  // whole warps past the end
+    const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x) / LANES, sub = lane % LANES;
+    if (i - lane / LANES >= nnode) return;  // whole warps past the end
     const bool live = i < nnode;
     const int row = live ? i : nnode - 1;
     const int d = live ? deg[row] : 0, first = IA[row];
-    const int64_t base = sell_ptr[row >> 5] + lane;
+    const int64_t base = sell_ptr[row >> 5] + (row & 31);
     const int steps = (int)((sell_ptr[(row >> 5) + 1] - sell_ptr[row >> 5]) / 32);
     double qi[5], D[25];
 #pragma unroll
@@ -692,6 +702,10 @@ __global__ void __launch_bounds__(32 * JAC_WARPS, MODE == 1 ? 2 : 3) k_jacobian(
         state_time_matrix(qi, f, D);
 #pragma unroll
         for (int k = 0; k < 25; k++) D[k] *= vd;
+    }
+    if (sub > 0) {
+#pragma unroll
+        for (int k = 0; k < 25; k++) D[k] = 0.0;
     }
     auto dissipation = [&](const double qL[5], const double qR[5], const double4 &g, double Ab[25]) {
         if (MODE == 1) {
@@ -723,7 +737,8 @@ __global__ void __launch_bounds__(32 * JAC_WARPS, MODE == 1 ? 2 : 3) k_jacobian(
         if constexpr (HIGH) stage[w][lane][k] = v;
         else store_low(&stage[w][lane][k], v);
     };
-    for (int k = 0; k < steps; k++) {
+    for (int k0 = 0; k0 < steps; k0 += LANES) {
+        const int k = k0 + sub;
         int slot = -1;
         if (k < d) {
             const int sn = sell_nbr[base + 32 * k];
@@ -757,7 +772,7 @@ __global__ void __launch_bounds__(32 * JAC_WARPS, MODE == 1 ? 2 : 3) k_jacobian(
         store(slot);
     }
     if (live)
-        for (int k = n2b_ptr[row]; k < n2b_ptr[row + 1]; k++) {
+        for (int k = n2b_ptr[row] + sub; k < n2b_ptr[row + 1]; k += LANES) {
             const int b = n2b[k];
             const int2 nd = bn[b];
             const double4 g = bg[b];
@@ -771,9 +786,13 @@ __global__ void __launch_bounds__(32 * JAC_WARPS, MODE == 1 ? 2 : 3) k_jacobian(
             for (int m = 0; m < 25; m++) D[m] += ha * (J[m] + Ab[m]);
         }
 #pragma unroll
+    for (int o = 1; o < LANES; o *= 2)
+#pragma unroll
+        for (int m = 0; m < 25; m++) D[m] += __shfl_xor_sync(0xffffffffu, D[m], o);
+#pragma unroll
     for (int m = 0; m < 25; m++) put(m, D[m]);
-    store(live ? IAU[row] : -1);
-    if (live) {
+    store(live && sub == 0 ? IAU[row] : -1);
+    if (live && sub == 0) {
 #pragma unroll
         for (int v = 0; v < 5; v++) {
             double r = res[v * (int64_t)nnode + row];
@@ -786,16 +805,23 @@ __global__ void __launch_bounds__(32 * JAC_WARPS, MODE == 1 ? 2 : 3) k_jacobian(
 // The approximate Roe Jacobian and right-hand side (MODE as k_jacobian).
 template <typename TA, int MODE>
 static void launch_jacobian(cfd_ctx *c, int add_time, int include_diss, double *A64, TA *Alow) {
-    auto run = [&](auto kern) {
-        kern<<<grid_for(c->nnode, 32 * JAC_WARPS), 32 * JAC_WARPS, 0, c->stream>>>(
+    auto run = [&](auto kern, int lanes) {
+        kern<<<grid_for((int64_t)c->nnode * lanes, 32 * JAC_WARPS), 32 * JAC_WARPS, 0, c->stream>>>(
             c->nnode, c->ldq, c->Q.p, c->IA.p, c->IAU.p, c->sell_ptr.p, c->sell_nbr.p, c->sell_geo.p, c->deg.p,
             c->n2b_ptr.p, c->n2b.p, c->bedge_nodes.p, c->bedge_geo.p, c->cvol.p, c->dt.p, c->res.p, c->resd.p,
             add_time, include_diss, c->flow, A64, Alow, c->B.p);
     };
-    const bool rup = c->flow.rup != 0;
-    if (A64 && Alow) run(rup ? k_jacobian<TA, MODE, true, true, true> : k_jacobian<TA, MODE, false, true, true>);
-    else if (A64) run(rup ? k_jacobian<TA, MODE, true, true, false> : k_jacobian<TA, MODE, false, true, false>);
-    else run(rup ? k_jacobian<TA, MODE, true, false, true> : k_jacobian<TA, MODE, false, false, true>);
+    const bool rup = c->flow.rup != 0, split = c->nnode <= kJacLanesRows;
+    if (A64 && Alow)
+        run(rup ? k_jacobian<TA, MODE, true, true, true, 4> : k_jacobian<TA, MODE, false, true, true, 4>, 4);
+    else if (A64 && split)
+        run(rup ? k_jacobian<TA, MODE, true, true, false, 4> : k_jacobian<TA, MODE, false, true, false, 4>, 4);
+    else if (A64)
+        run(rup ? k_jacobian<TA, MODE, true, true, false, 1> : k_jacobian<TA, MODE, false, true, false, 1>, 1);
+    else if (split)
+        run(rup ? k_jacobian<TA, MODE, true, false, true, 4> : k_jacobian<TA, MODE, false, false, true, 4>, 4);
+    else
+        run(rup ? k_jacobian<TA, MODE, true, false, true, 1> : k_jacobian<TA, MODE, false, false, true, 1>, 1);
 }
 
 template <typename TA>
