@@ -91,6 +91,7 @@ struct Abmc {
     bool built = false;
     int ncolor = 0, maxrow = 0, maxstage = 0, maxblk = 0, maxpairs = 0, stage = 0;
     bool by_cta = false;              // patches fit the CTA-per-patch factorisation
+    double levels = 0.0;              // mean levels of a patch's rows
     std::vector<int> cptr;            // host [ncolor+1] into patches
     std::vector<int> h_pcolor;        // host colour of each patch
     DevBuf<int> patches;              // patch ids in colour order

@@ -187,10 +187,11 @@ __host__ __device__ inline size_t mc_factor_warp_bytes(int maxrow, int maxstage)
 // loc[k] is the place of CRS block k, meta[i].w = level of row i in its patch |
 // pairs of its off-patch blocks << 8.
 // hdr[IA[i]+u] = (place of inv(U_pp), pairs, CRS-local slot of (i,p), 0);
-// pairs are (place of U_pj, CRS-local slot of (i,j)).  For p in row i's patch
-// the places are CRS positions in the patch instead, and hdr.w is p's level.
+// pairs are (place of U_pj, CRS-local slot of (i,j)).  Where the CTA-per-patch
+// kernel can run too (by_cta), the places of blocks of p in row i's own patch
+// are CRS positions in the patch instead, and hdr.w is p's level.
 template <typename TA, typename TM>
-__global__ void k_mc_factor(const int *__restrict__ patches, int npatch, int n, int maxrow, int maxstage,
+__global__ void k_mc_factor(const int *__restrict__ patches, int npatch, int n, int maxrow, int maxstage, int by_cta,
                             const int *__restrict__ IA, const int *__restrict__ slot, const int4 *__restrict__ meta,
                             const int4 *__restrict__ hdr, const unsigned *__restrict__ loc,
                             const int64_t *__restrict__ pair_ptr, const int2 *__restrict__ pairs,
@@ -221,13 +222,12 @@ __global__ void k_mc_factor(const int *__restrict__ patches, int npatch, int n, 
             for (int e = lane; e < nlo; e += 32) {
                 const int4 h = hdr[base + e];
                 hd[e] = h;
-                // blocks of the patch's own rows are named by their position in it
-                src[e] = e < mt.x ? h.x : (int)loc[base0 + h.x];
+                src[e] = !by_cta || e < mt.x ? h.x : (int)loc[base0 + h.x];
             }
             for (int e = lane; e < npair; e += 32) {
                 const int2 pr = pairs[pp + e];
                 pm[e] = pr.y;
-                src[nlo + e] = e < next_pairs ? pr.x : (int)loc[base0 + pr.x];
+                src[nlo + e] = !by_cta || e < next_pairs ? pr.x : (int)loc[base0 + pr.x];
             }
             for (int e = lane; e < len; e += 32) sl[e] = slot[base + e] - base;
             // one block per lane, its 25 loads in flight together
@@ -252,10 +252,27 @@ __global__ void k_mc_factor(const int *__restrict__ patches, int npatch, int n, 
             int t0 = 0;
             for (int u = 0; u < nlo; u++) {
                 const int4 h = hd[u];
-                const TM *iv = stg + u * 25, *Up = stg + (size_t)(nlo + t0) * 25;
-                const int *to = pm + t0;
-                mc_eliminate(w, h.z, h.y, [&](int t) { return to[t]; }, [&](int k) { return (double)iv[k]; },
-                             [&](int t, int k) { return (double)Up[t * 25 + k]; }, lane);
+                const int tk = h.z;
+                // L_ip = A_ip inv(U_pp)
+                double Lab = 0.0;
+                if (lane < 25) {
+#pragma unroll
+                    for (int c = 0; c < 5; c++) Lab = fma(w[tk * 25 + a * 5 + c], (double)stg[u * 25 + c * 5 + b], Lab);
+                }
+                __syncwarp();
+                if (lane < 25) w[tk * 25 + lane] = Lab;
+                __syncwarp();
+                // A_ij -= L_ip U_pj, the pairs' 25 entries spread over the lanes
+                for (int e = lane; e < h.y * 25; e += 32) {
+                    const int t = e / 25, ab = e - 25 * t, ea = ab / 5, eb = ab - 5 * ea;
+                    const int mj = pm[t0 + t];
+                    const TM *U = stg + (size_t)(nlo + t0 + t) * 25;
+                    double s = w[mj * 25 + ab];
+#pragma unroll
+                    for (int c = 0; c < 5; c++) s = fma(-w[tk * 25 + ea * 5 + c], (double)U[c * 5 + eb], s);
+                    w[mj * 25 + ab] = s;
+                }
+                __syncwarp();
                 t0 += h.y;
             }
             const int td = sl[nlo];  // the diagonal follows the lower entries
@@ -267,9 +284,14 @@ __global__ void k_mc_factor(const int *__restrict__ patches, int npatch, int n, 
                 if (lane < 25) w[td * 25 + lane] = iv;
             }
             __syncwarp();
-            for (int e = lane; e < len * 25; e += 32) {
-                const int u = e / 25, rc = e - 25 * u;
-                st<TM>(M + mc_element(loc[base + sl[u]], rc / 5, rc % 5), w[sl[u] * 25 + rc]);
+            // a block per step, an entry per lane, the places of eight blocks in flight
+            for (int t8 = 0; t8 < len; t8 += 8) {
+                unsigned to[8];
+#pragma unroll
+                for (int k = 0; k < 8; k++) to[k] = loc[base + min(t8 + k, len - 1)];
+#pragma unroll
+                for (int k = 0; k < 8; k++)
+                    if (t8 + k < len && lane < 25) st<TM>(M + mc_element(to[k], a, b), w[(t8 + k) * 25 + lane]);
             }
             __syncwarp();
         }
@@ -278,26 +300,25 @@ __global__ void k_mc_factor(const int *__restrict__ patches, int npatch, int n, 
 
 // Factorisation of the patches of one colour, one CTA of 16 warps per patch:
 // the same operations as the warp-per-patch kernel, for meshes whose patches'
-// blocks fit in shared memory in FP64 (and see kMcWarpPatches).  The patch's blocks and lists are
-// loaded once.  Blocks that couple to other patches come first in every row's
-// order and depend on nothing inside the patch, so the warps, two rows each,
-// eliminate them at once, staging the factor blocks of the other patches.
-// Then, level by level, the rows of a level invert their diagonal blocks, and
-// every row eliminates its blocks in their columns.
+// blocks fit in shared memory in FP64 (and see mc_factor_by_cta).  The patch's
+// blocks and lists are loaded once.  Blocks that couple to other patches come
+// first in every row's order and depend on nothing inside the patch, so the
+// warps, two rows each, eliminate them at once, staging the factor blocks of
+// the other patches.  Then, level by level, the rows of a level invert their
+// diagonal blocks, and every row eliminates its blocks in their columns.
 // Bound by the chain of a patch's levels, some 9 inversions and eliminations
-// behind each other, where the warp-per-patch kernel takes 32 rows one after
-// the other.  A cfd_gmres call of one iteration (factorisation, two applies) on
-// the tet cubes, FP32 / FP64: 24^3 0.91 / 0.98 ms, 48^3 2.1 / 2.3, 64^3 4.0 /
-// 4.4, 96^3 11.5 / 12.8; with the warp-per-patch kernel 4.0 / 4.6, 5.2 / 5.8,
-// 6.5 / 7.4 and 12.6 / 15.4 ms.
+// behind each other (up to 32 on a mesh numbered along its lines), where the
+// warp-per-patch kernel takes 32 rows one after the other.  A cfd_gmres call of
+// one iteration (factorisation, two applies) with a CTA / a warp per patch, FP32
+// factors: tets in blocked RCM order 24^3 0.77 / 3.8 ms, 64^3 3.7 / 6.2, 96^3
+// 10.7 / 11.3, 112^3 16.8 / 14.4; in natural order 40^3 1.7 / 2.9, 64^3 5.6 /
+// 4.0; hexahedra in blocked RCM order 64^3 2.3 / 2.5, 96^3 6.6 / 4.5, in natural
+// order 40^3 1.16 / 0.86, 96^3 13.0 / 4.0.  FP64: tets 96^3 11.7 / 13.6, in
+// natural order 17.9 / 13.5, hexahedra 6.8 / 5.2.  By the rule: 10.7 and 13.5 ms
+// for the tets of 96^3 and 112^3 in FP32, 4.2 for the hexahedra of 96^3.
 constexpr int kMcFactorWarps = 16, kMcFactorRows = kMcRows / kMcFactorWarps;
 static_assert(kMcFactorRows == 2, "two rows per warp");
 constexpr size_t kMcFactorBytes = 222u << 10;  // its shared memory at most
-// FP32 factors of colours with more patches per SM than this go to the warp
-// kernel, whose twenty warps per SM are then all busy: 128^3 cube (41 patches per
-// SM and colour) 22.3 ms per call, 26.1 with a CTA per patch; 96^3 (18) 12.6 and
-// 11.5.  FP64 factors leave it fewer warps: 33.3 and 29.1 ms at 128^3.
-constexpr int kMcWarpPatches = 28;
 __host__ __device__ inline size_t mc_factor_cta_bytes(int maxblk, int maxpairs) {
     return ((size_t)maxblk * (25 * sizeof(double) + sizeof(int4) + 2 * sizeof(int)) + (size_t)maxpairs * sizeof(int2) + 15) &
            ~(size_t)15;
@@ -919,6 +940,13 @@ int mc_build(cfd_ctx *c) {
             meta[i].w = l;
         }
     });
+    int64_t levels = 0;
+    for (int P = 0; P < np; P++) {
+        int l = 0;
+        for (int i = P * kMcRows; i < std::min(n, (P + 1) * kMcRows); i++) l = std::max(l, meta[i].w);
+        levels += l + 1;
+    }
+    mc.levels = (double)levels / np;
     int maxblk = 0;
     for (int P = 0; P < np; P++) maxblk = std::max(maxblk, IA[std::min(n, (P + 1) * kMcRows)] - IA[P * kMcRows]);
     // The solves' plan of each patch and direction (0 forward, 1 backward):
@@ -1078,6 +1106,7 @@ int mc_build(cfd_ctx *c) {
     // binary search, JA rows being sorted).  Counted, then written, per row.
     std::vector<int4> hdr(c->nnzb, make_int4(0, 0, 0, 0));
     std::vector<int> ext_pairs(n, 0);  // pairs of each row's off-patch blocks
+    std::vector<int> ext_most(n, 0);   // and the most of one such block
     std::vector<int64_t> pair_ptr(n + 1, 0);
     auto row_pairs = [&](int i, int2 *out) {  // returns the row's pair count; writes them when out != nullptr
         const int base = IA[i], end = IA[i + 1];
@@ -1085,24 +1114,25 @@ int mc_build(cfd_ctx *c) {
         int total = 0, next_pairs = 0;
         for (int u = 0; u < nlo; u++) {
             const int kk = slot[base + u], p = JA[kk];
-            // blocks of the patch's own rows are named by their CRS position in the patch
-            const bool own = u >= meta[i].x;
+            // see k_mc_factor: blocks of the patch's own rows are named by their CRS position in the patch
+            const bool own = u >= meta[i].x, named = own && mc.by_cta;
             const int patch0 = IA[i / kMcRows * kMcRows];
             int cnt = 0;
             for (int v = IA[p] + meta[p].y + 1; v < IA[p + 1]; v++) {
                 const int j = scol[v];
                 const int *it = std::lower_bound(&JA[base], &JA[0] + end, j);
                 if (it != &JA[0] + end && *it == j) {
-                    if (out) out[total + cnt] = make_int2(own ? slot[v] - patch0 : (int)loc[v], (int)(it - &JA[base]));
+                    if (out) out[total + cnt] = make_int2(named ? slot[v] - patch0 : (int)loc[v], (int)(it - &JA[base]));
                     cnt++;
                 }
             }
             if (out) {
                 const int dg = IA[p] + meta[p].y;  // the diagonal's list entry
-                hdr[base + u] = make_int4(own ? slot[dg] - patch0 : (int)loc[dg], cnt, kk - base,
+                hdr[base + u] = make_int4(named ? slot[dg] - patch0 : (int)loc[dg], cnt, kk - base,
                                           own ? meta[p].w & 255 : 0);
                 if (!own) next_pairs += cnt;
             }
+            if (!out && !own) ext_most[i] = std::max(ext_most[i], cnt);
             total += cnt;
         }
         // other threads read the level meanwhile: the counts go in afterwards
@@ -1120,21 +1150,17 @@ int mc_build(cfd_ctx *c) {
     int64_t maxpairs = 1;
     for (int P = 0; P < np; P++)
         maxpairs = std::max(maxpairs, pair_ptr[std::min(n, (P + 1) * kMcRows)] - pair_ptr[P * kMcRows]);
+    // the CTA-per-patch factorisation, when its patches fit in either precision
+    mc.maxblk = maxblk;
+    mc.maxpairs = (int)std::min<int64_t>(maxpairs, 1 << 24);
+    mc.stage = std::max(24, 1 + *std::max_element(ext_most.begin(), ext_most.end()));
+    mc.by_cta = mc_factor_cta_bytes(mc.maxblk, mc.maxpairs) + (size_t)kMcFactorWarps * mc.stage * 25 * sizeof(double) <=
+                kMcFactorBytes;
     std::vector<int2> pairs(std::max<int64_t>(pair_ptr[n], 1));
     parallel_rows([&](int i0, int i1) {
         for (int i = i0; i < i1; i++) row_pairs(i, pairs.data() + pair_ptr[i]);
     });
-    int maxcnt = 0;
-    for (int i = 0; i < n; i++) {
-        meta[i].w |= ext_pairs[i] << 8;
-        for (int u = IA[i]; u < IA[i] + meta[i].x; u++) maxcnt = std::max(maxcnt, hdr[u].y);
-    }
-    // the CTA-per-patch factorisation, when its patches fit in either precision
-    mc.maxblk = maxblk;
-    mc.maxpairs = (int)std::min<int64_t>(maxpairs, 1 << 24);
-    mc.stage = std::max(24, 1 + maxcnt);
-    mc.by_cta = mc_factor_cta_bytes(mc.maxblk, mc.maxpairs) + (size_t)kMcFactorWarps * mc.stage * 25 * sizeof(double) <=
-                kMcFactorBytes;
+    for (int i = 0; i < n; i++) meta[i].w |= ext_pairs[i] << 8;
     mc.maxrow = maxrow;
     mc.maxstage = maxstage;
     CFD_CUDA(mc.patches.upload(patches.data(), patches.size(), c->stream));
@@ -1151,6 +1177,18 @@ int mc_build(cfd_ctx *c) {
     CFD_CUDA(stream_wait(c->stream));  // host vectors go out of scope
     mc.built = true;
     return CFD_OK;
+}
+
+// Whether a colour of cnt patches is factored by a CTA per patch, from measured
+// costs per colour (microseconds; p patches per SM, b blocks per row, l levels
+// per patch): p (2.3 b + 1.7 l) with a CTA per patch, whose levels follow one
+// another; with a warp per patch 26-30 b for its 32 rows, whatever p, and from
+// some 15 patches per SM, when its twenty warps are busy, 3.2 b p with FP32 and
+// 4.1 b p with FP64 factors (fewer warps fit).
+static bool mc_factor_by_cta(const cfd_ctx *c, int cnt, size_t elem) {
+    const Abmc &mc = c->mc;
+    const double b = (double)c->nnzb / c->nnode, p = (double)cnt / c->nsm;
+    return mc.by_cta && (p * (b + 1.7 * mc.levels) <= 30.0 * b || (elem == 8 && 1.7 * mc.levels <= 1.3 * b));
 }
 
 template <typename TA, typename TM>
@@ -1182,14 +1220,13 @@ int mc_factor(cfd_ctx *c, const TA *A, TM *M) {
     CFD_CUDA(allow_max_dynamic_smem(k_mc_factor_cta<TA, TM>, c->device, &smax));
     for (int k = 0; k < mc.ncolor; k++) {
         const int cnt = mc.cptr[k + 1] - mc.cptr[k];
-        const bool many = sizeof(TM) == 4 && cnt > kMcWarpPatches * c->nsm;
-        if (mc.by_cta && smem_cta <= (size_t)smax && !many)
+        if (smem_cta <= (size_t)smax && mc_factor_by_cta(c, cnt, sizeof(TM)))
             k_mc_factor_cta<TA, TM><<<cnt, 32 * kMcFactorWarps, smem_cta, c->stream>>>(
                 mc.patches.p + mc.cptr[k], c->nnode, mc.maxblk, mc.maxpairs, mc.stage, c->IA.p, mc.slot.p, mc.meta.p,
                 mc.hdr.p, mc.loc.p, mc.pair_ptr.p, mc.pairs.p, A, M, c->err.p);
         else
             k_mc_factor<TA, TM><<<grid_for(cnt, nwarp), 32 * nwarp, smem, c->stream>>>(
-                mc.patches.p + mc.cptr[k], cnt, c->nnode, mc.maxrow, mc.maxstage, c->IA.p, mc.slot.p, mc.meta.p,
+                mc.patches.p + mc.cptr[k], cnt, c->nnode, mc.maxrow, mc.maxstage, mc.by_cta, c->IA.p, mc.slot.p, mc.meta.p,
                 mc.hdr.p, mc.loc.p, mc.pair_ptr.p, mc.pairs.p, A, M, c->err.p);
     }
     CFD_LAUNCH_CHECK();
