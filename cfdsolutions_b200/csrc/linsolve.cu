@@ -395,25 +395,28 @@ __global__ void k_sub(int64_t n, const double *__restrict__ b, const double *__r
 // multiplying column c of each 5x5 block: a block costs a lane one value of x
 // and five entries of A, each load of five lanes contiguous, where a lane that
 // owns an output loads all five values of x and a strided row of the block.
-// Five blocks are in flight per lane; the column ids are loaded two such
+// Four blocks are in flight per lane; the column ids are loaded two such
 // batches ahead and the values of x one ahead, so that no load waits for
 // another one.  The partial outputs are added across the five lanes through
 // shared memory at the end of the row.
-// Measured on the 96^3 cube (0.91 M rows, 13.5 M blocks), of 6.45 TB/s: FP32
-// 281 us, 5.3 TB/s (336 us with a lane per output; 320 without the ids and
-// values ahead), FP64 436 us, 6.4 TB/s (482): bound by DRAM.  Slower: the CTA's
-// blocks staged in shared memory by 16-byte copies (320-348 us, FP32: fewer
-// warps), prefetching a later CTA's blocks into L2 (379 us).
+// Measured of 6.45 TB/s, tets 96^3 (0.91 M rows, 13.5 M blocks): FP32 270 us, 5.5
+// TB/s (336 us with a lane per output; 320 without the ids and values ahead),
+// FP64 424 us, 6.6 TB/s (482), BF16 254 (326); hexahedra 96^3 (6.3 M blocks): 154,
+// 229 and 144 us (with a lane per output 164, 240 and 148).  Bound by DRAM.  Five
+// blocks in flight take 72 registers and leave a batch that rows of 7 blocks
+// fill badly: tets 281, 437, 269 us, hexahedra 172, 257, 162; three: tets 276, 429,
+// 264, hexahedra 161, 234, 147.  Slower: the CTA's blocks staged in shared memory
+// by 16-byte copies (320-348 us, tets FP32: fewer warps), prefetching a later
+// CTA's blocks into L2 (379 us).
 template <typename TA>
 __device__ __forceinline__ double ldA(const TA *p);
 template <>
 __device__ __forceinline__ double ldA<double>(const double *p) { return __ldg(p); }
 template <>
 __device__ __forceinline__ double ldA<float>(const float *p) { return (double)__ldg(p); }
-template <>
-__device__ __forceinline__ double ldA<uint16_t>(const uint16_t *p) { return load_low(p); }
 
 constexpr int kSpmvWarps = 4, kSpmvRows = 6 * kSpmvWarps, kSpmvThreads = 32 * kSpmvWarps;
+constexpr int kSpmvBatch = 4;  // blocks in flight per lane, at most 5
 // The block SpMV of rows kSpmvRows * cta .. of one CTA.
 template <typename TA>
 __device__ __forceinline__ void bspmv_cta(int cta, int nrow, const int *__restrict__ IA, const int *__restrict__ JA,
@@ -430,30 +433,30 @@ __device__ __forceinline__ void bspmv_cta(int cta, int nrow, const int *__restri
         int k = IA[r];
         const int k1 = IA[r + 1];
         const TA *a = A + (int64_t)k * 25 + c;
-        // column ids two batches of five blocks ahead, values of x one ahead
+        // column ids two batches of blocks ahead, values of x one ahead
         auto ids = [&](int at) { return at + c < k1 ? JA[at + c] : 0; };
-        auto values = [&](int j, double v[5]) {
+        auto values = [&](int j, double v[kSpmvBatch]) {
 #pragma unroll
-            for (int t = 0; t < 5; t++) v[t] = __ldg(x + (int64_t)__shfl_sync(group, j, 5 * g + t) * 5 + c);
+            for (int t = 0; t < kSpmvBatch; t++) v[t] = __ldg(x + (int64_t)__shfl_sync(group, j, 5 * g + t) * 5 + c);
         };
-        double xv[5];
-        int j1 = ids(k), j2 = ids(k + 5);
+        double xv[kSpmvBatch];
+        int j1 = ids(k), j2 = ids(k + kSpmvBatch);
         values(j1, xv);
-        for (; k + 5 <= k1; k += 5, a += 125) {
-            double av[25], xn[5];
+        for (; k + kSpmvBatch <= k1; k += kSpmvBatch, a += 25 * kSpmvBatch) {
+            double av[5 * kSpmvBatch], xn[kSpmvBatch];
 #pragma unroll
-            for (int t = 0; t < 25; t++) av[t] = load_low(a + 5 * t);
+            for (int t = 0; t < 5 * kSpmvBatch; t++) av[t] = load_low(a + 5 * t);
             values(j2, xn);
-            j2 = ids(k + 10);
+            j2 = ids(k + 2 * kSpmvBatch);
 #pragma unroll
-            for (int t = 0; t < 5; t++)
+            for (int t = 0; t < kSpmvBatch; t++)
 #pragma unroll
                 for (int m = 0; m < 5; m++) acc[m] = fma(av[5 * t + m], xv[t], acc[m]);
 #pragma unroll
-            for (int t = 0; t < 5; t++) xv[t] = xn[t];
+            for (int t = 0; t < kSpmvBatch; t++) xv[t] = xn[t];
         }
 #pragma unroll
-        for (int t = 0; t < 4; t++)
+        for (int t = 0; t < kSpmvBatch - 1; t++)
             if (k + t < k1) {
 #pragma unroll
                 for (int m = 0; m < 5; m++) acc[m] = fma(load_low(a + 25 * t + 5 * m), xv[t], acc[m]);
