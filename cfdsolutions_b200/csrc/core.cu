@@ -697,11 +697,15 @@ __global__ void __launch_bounds__(32 * JAC_WARPS, MODE == 1 ? 2 : 3) k_jacobian(
         pc_node_cinv(qi, f, D);
 #pragma unroll
         for (int k = 0; k < 25; k++) D[k] *= vd;
-    } else {
+    } else if (RUP) {
         // (V/dt) dQ/dW
         state_time_matrix(qi, f, D);
 #pragma unroll
         for (int k = 0; k < 25; k++) D[k] *= vd;
+    } else {
+        // no product with the zeros of the identity: V/dt may be infinite
+#pragma unroll
+        for (int k = 0; k < 25; k++) D[k] = k % 6 == 0 ? vd : 0.0;
     }
     if (sub > 0) {
 #pragma unroll
