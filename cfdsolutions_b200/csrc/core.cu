@@ -645,7 +645,11 @@ __global__ void k_add_diss(int64_t n, const double *__restrict__ a, const double
 // us (58 / 61).  Bound by latency at three CTAs per SM (168 registers).  The
 // lanes stage their blocks in shared memory and the warp stores them one after
 // the other, 100 or 200 contiguous bytes each; a row's next block follows in
-// the next step, so the sectors they share fill in L2.
+// the next step, so the sectors they share fill in L2.  Eight of these stores
+// in flight suit BF16 blocks and Thornber's form (BF16, 66^3 cube: Thornber 534 /
+// 494 us with four / eight, Roe 413 / 397; 16: 515 and 406), four the others
+// (FP32 Roe 386 / 408); two matrices are stored by all 32 lanes (617 us, 642 with
+// a block per step).
 // The low-precision-only system sums the diagonal from the rounded blocks.
 // MODE: 0 Roe, 1 preconditioned Roe (CFD_FLUX_ROE_PRECOND), 2 Thornber (|A| of
 // the modified states).  RUP: the state's variables (f.rup).  HIGH / LOW: an
@@ -657,9 +661,11 @@ constexpr int JAC_WARPS = 4;  // warps per CTA
 // works off its edges one behind the other: 8^3 cube (729 rows), Roe FP64 39.5 /
 // 14.9 us with 1 / 4 lanes, preconditioned Roe 78.9 / 29.2, 24^3 (15,625 rows)
 // 41.4 / 33.2 and 80.4 / 64.2; 64^3 FP32 347 / 377, preconditioned 724 / 865.
-// With two matrices stored, FP64 and a low-precision one, four lanes are the
-// faster at every size but small boxes of hexahedra (tets 24^3 70 / 49 us, 48^3
-// 346 / 269, 80^3 1300 / 1128; hexahedra 32^3 41 / 48, 64^3 324 / 332).
+// With two matrices stored, FP64 and a low-precision one, it is four lanes up to
+// the same limit and two above (Roe, FP64 and FP32, 4 / 2 lanes: tets 20^3 25.2 /
+// 32.8 us, 26^3 53.7 / 46.8, 48^3 255 / 271, 66^3 617 / 627, preconditioned 1063 /
+// 887; hexahedra, whose rows have six edges, 16^3 12.7 / 16.7, 32^3 38.3 / 35.4,
+// 96^3 977 / 844; a thread per row: tets 24^3 70, 48^3 346).
 constexpr int kJacLanesRows = 16000;
 
 template <typename TA>
@@ -679,6 +685,7 @@ __global__ void __launch_bounds__(32 * JAC_WARPS, MODE == 1 ? 2 : 3) k_jacobian(
     int include_diss, Flow f, double *__restrict__ A64, TA *__restrict__ Alow, double *__restrict__ B) {
     f.rup = RUP ? 1 : 0;  // a compile-time constant below
     using TS = std::conditional_t<HIGH, double, TA>;  // staged blocks
+    constexpr int kUnroll = sizeof(TS) == 2 || MODE == 2 ? 8 : 4;  // of the stores
     __shared__ TS stage[JAC_WARPS][32][25];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x) / LANES, sub = lane % LANES;
@@ -722,16 +729,29 @@ __global__ void __launch_bounds__(32 * JAC_WARPS, MODE == 1 ? 2 : 3) k_jacobian(
             roe_abs_jacobian(qL, qR, g.x, g.y, g.z, f, Ab);
         }
     };
-    // the warp's staged blocks to their slots, lane m element m; slot < 0: none
+    // the warp's staged blocks to their slots; slot < 0: none
     auto store = [&](int slot) {
         __syncwarp();
-        for (int b = 0; b < 32; b++) {
-            const int at = __shfl_sync(0xffffffffu, slot, b);
-            if (at < 0 || lane >= 25) continue;
-            const TS v = stage[w][b][lane];
-            if (HIGH) A64[(int64_t)at * 25 + lane] = v;
-            if (LOW) {
-                if constexpr (HIGH) store_low(Alow + (int64_t)at * 25 + lane, v);
+        if constexpr (HIGH && LOW) {
+            // all 32 lanes, 800 elements as they lie
+#pragma unroll 5
+            for (int k = 0; k < 25; k++) {
+                const int e = lane + 32 * k, b = e / 25;
+                const int at = __shfl_sync(0xffffffffu, slot, b);
+                const TS v = stage[w][b][e - 25 * b];
+                if (at < 0) continue;
+                const int64_t to = (int64_t)at * 25 + (e - 25 * b);
+                A64[to] = v;
+                store_low(Alow + to, v);
+            }
+        } else {
+            // a block per step, lane m element m
+#pragma unroll(kUnroll)
+            for (int b = 0; b < 32; b++) {
+                const int at = __shfl_sync(0xffffffffu, slot, b);
+                if (at < 0 || lane >= 25) continue;
+                const TS v = stage[w][b][lane];
+                if constexpr (HIGH) A64[(int64_t)at * 25 + lane] = v;
                 else Alow[(int64_t)at * 25 + lane] = v;
             }
         }
@@ -816,8 +836,10 @@ static void launch_jacobian(cfd_ctx *c, int add_time, int include_diss, double *
             add_time, include_diss, c->flow, A64, Alow, c->B.p);
     };
     const bool rup = c->flow.rup != 0, split = c->nnode <= kJacLanesRows;
-    if (A64 && Alow)
+    if (A64 && Alow && split)
         run(rup ? k_jacobian<TA, MODE, true, true, true, 4> : k_jacobian<TA, MODE, false, true, true, 4>, 4);
+    else if (A64 && Alow)
+        run(rup ? k_jacobian<TA, MODE, true, true, true, 2> : k_jacobian<TA, MODE, false, true, true, 2>, 2);
     else if (A64 && split)
         run(rup ? k_jacobian<TA, MODE, true, true, false, 4> : k_jacobian<TA, MODE, false, true, false, 4>, 4);
     else if (A64)
