@@ -23,6 +23,7 @@
 #include <atomic>
 #include <cstdint>
 #include <cstring>
+#include <memory>
 #include <set>
 #include <tuple>
 #include <vector>
@@ -1090,27 +1091,32 @@ int mc_build(cfd_ctx *c) {
             set_error("ILU(0) multicolour: patch lists too long");
             return CFD_ERR_RANGE;
         }
-        std::vector<unsigned char> all(words * 16);
+        std::unique_ptr<unsigned char[]> all(new unsigned char[words * 16]);  // every byte written below
         parallel_patches([&](int, int64_t q0, int64_t q1) {
             for (int pos = (int)q0; pos < (int)q1; pos++)
-                std::memcpy(all.data() + (size_t)desc[dir][pos].x * 16, lists[dir][pos].data(), lists[dir][pos].size());
+                std::memcpy(all.get() + (size_t)desc[dir][pos].x * 16, lists[dir][pos].data(), lists[dir][pos].size());
         });
         CFD_CUDA(mc.desc[dir].upload(desc[dir].data(), desc[dir].size(), c->stream));
-        CFD_CUDA(mc.lists[dir].upload(reinterpret_cast<const uint4 *>(all.data()), words, c->stream));
+        CFD_CUDA(mc.lists[dir].upload(reinterpret_cast<const uint4 *>(all.get()), words, c->stream));
         CFD_CUDA(stream_wait(c->stream));
     }
     // update lists of the factorisation: for lower block (i,p), the upper
     // blocks (p,j) of row p whose column j row i also holds
     // Row i's pairs in order: for each lower block u, the upper entries v of
-    // row p = JA[slot[base+u]] whose column row i holds (its CRS-local slot by
-    // binary search, JA rows being sorted).  Counted, then written, per row.
-    std::vector<int4> hdr(c->nnzb, make_int4(0, 0, 0, 0));
+    // row p = JA[slot[base+u]] whose column row i holds, with its CRS-local slot.
+    // Counted, then written, per row.  local[j] = that slot of column j, -1 outside
+    // the call (searching the row for each column took three times as long).
+    // hdr and pairs are written whole by the rows' threads (zeroing 500 MB each at
+    // 128^3 on one thread took longer than the lists themselves)
+    std::unique_ptr<int4[]> hdr(new int4[c->nnzb]);
     std::vector<int> ext_pairs(n, 0);  // pairs of each row's off-patch blocks
     std::vector<int> ext_most(n, 0);   // and the most of one such block
     std::vector<int64_t> pair_ptr(n + 1, 0);
-    auto row_pairs = [&](int i, int2 *out) {  // returns the row's pair count; writes them when out != nullptr
+    // returns the row's pair count; writes the pairs and headers when out != nullptr
+    auto row_pairs = [&](int i, int2 *out, std::vector<int> &local) {
         const int base = IA[i], end = IA[i + 1];
         const int nlo = meta[i].y;
+        for (int k = end - 1; k >= base; k--) local[JA[k]] = k - base;
         int total = 0, next_pairs = 0;
         for (int u = 0; u < nlo; u++) {
             const int kk = slot[base + u], p = JA[kk];
@@ -1119,12 +1125,10 @@ int mc_build(cfd_ctx *c) {
             const int patch0 = IA[i / kMcRows * kMcRows];
             int cnt = 0;
             for (int v = IA[p] + meta[p].y + 1; v < IA[p + 1]; v++) {
-                const int j = scol[v];
-                const int *it = std::lower_bound(&JA[base], &JA[0] + end, j);
-                if (it != &JA[0] + end && *it == j) {
-                    if (out) out[total + cnt] = make_int2(named ? slot[v] - patch0 : (int)loc[v], (int)(it - &JA[base]));
-                    cnt++;
-                }
+                const int l = local[scol[v]];
+                if (l < 0) continue;
+                if (out) out[total + cnt] = make_int2(named ? slot[v] - patch0 : (int)loc[v], l);
+                cnt++;
             }
             if (out) {
                 const int dg = IA[p] + meta[p].y;  // the diagonal's list entry
@@ -1135,12 +1139,15 @@ int mc_build(cfd_ctx *c) {
             if (!out && !own) ext_most[i] = std::max(ext_most[i], cnt);
             total += cnt;
         }
+        for (int k = base; k < end; k++) local[JA[k]] = -1;
+        if (out) std::fill(hdr.get() + base + nlo, hdr.get() + end, make_int4(0, 0, 0, 0));
         // other threads read the level meanwhile: the counts go in afterwards
         if (out) ext_pairs[i] = next_pairs;
         return total;
     };
     parallel_rows([&](int i0, int i1) {
-        for (int i = i0; i < i1; i++) pair_ptr[i + 1] = row_pairs(i, nullptr);
+        std::vector<int> local(n, -1);
+        for (int i = i0; i < i1; i++) pair_ptr[i + 1] = row_pairs(i, nullptr, local);
     });
     int maxstage = 1;
     for (int i = 0; i < n; i++) {
@@ -1156,9 +1163,10 @@ int mc_build(cfd_ctx *c) {
     mc.stage = std::max(24, 1 + *std::max_element(ext_most.begin(), ext_most.end()));
     mc.by_cta = mc_factor_cta_bytes(mc.maxblk, mc.maxpairs) + (size_t)kMcFactorWarps * mc.stage * 25 * sizeof(double) <=
                 kMcFactorBytes;
-    std::vector<int2> pairs(std::max<int64_t>(pair_ptr[n], 1));
+    std::unique_ptr<int2[]> pairs(new int2[std::max<int64_t>(pair_ptr[n], 1)]);
     parallel_rows([&](int i0, int i1) {
-        for (int i = i0; i < i1; i++) row_pairs(i, pairs.data() + pair_ptr[i]);
+        std::vector<int> local(n, -1);
+        for (int i = i0; i < i1; i++) row_pairs(i, pairs.get() + pair_ptr[i], local);
     });
     for (int i = 0; i < n; i++) meta[i].w |= ext_pairs[i] << 8;
     mc.maxrow = maxrow;
@@ -1171,9 +1179,9 @@ int mc_build(cfd_ctx *c) {
         for (int64_t u = u0; u < u1; u++) place[slot[u]] = loc[u];
     });
     CFD_CUDA(mc.loc.upload(place.data(), place.size(), c->stream));
-    CFD_CUDA(mc.hdr.upload(hdr.data(), hdr.size(), c->stream));
+    CFD_CUDA(mc.hdr.upload(hdr.get(), (size_t)c->nnzb, c->stream));
     CFD_CUDA(mc.pair_ptr.upload(pair_ptr.data(), pair_ptr.size(), c->stream));
-    CFD_CUDA(mc.pairs.upload(pairs.data(), (size_t)pair_ptr[n], c->stream));
+    CFD_CUDA(mc.pairs.upload(pairs.get(), (size_t)pair_ptr[n], c->stream));
     CFD_CUDA(stream_wait(c->stream));  // host vectors go out of scope
     mc.built = true;
     return CFD_OK;
