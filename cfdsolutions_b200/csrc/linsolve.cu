@@ -813,11 +813,13 @@ static int precond_apply(cfd_ctx *c, const Precond &pc, const double *r, double 
 static int spmv(cfd_ctx *c, int prec, const double *x, double *y) {
     const int n = c->nnode;
     const int g = spmv_blocks(n), b = kSpmvThreads;
+    // the copies of this system: FP64 unless a64_valid says no, and a_precision;
+    // what else is allocated belongs to an earlier system
+    if (prec != c->a_precision) prec = CFD_PREC_FP64;
     if (prec == CFD_PREC_FP64 && !c->a64_valid) prec = c->a_precision;  // low-precision-only system
-    const void *A = prec == CFD_PREC_FP32 && c->A32.p   ? (const void *)c->A32.p
-                    : prec == CFD_PREC_BF16 && c->A16.p ? (const void *)c->A16.p
-                                                        : (const void *)c->A64.p;
-    if (A == c->A64.p) prec = CFD_PREC_FP64;
+    const void *A = prec == CFD_PREC_FP32   ? (const void *)c->A32.p
+                    : prec == CFD_PREC_BF16 ? (const void *)c->A16.p
+                                            : (const void *)c->A64.p;
     if (c->batcher) {
         // the serving loop fuses this launch with other requests' (bit-identical per row)
         const SpmvJob job{n, c->IA.p, c->JA.p, A, x, y, 0};
