@@ -472,16 +472,68 @@ __device__ __forceinline__ void bspmv_cta(int cta, int nrow, const int *__restri
     }
 }
 
+// The same for matrices of short rows (see spmv_by_output): five lanes per row
+// without idle ones, lane m forming output m from row m of each block, two
+// blocks per step with their own partial sums.
 template <typename TA>
+__device__ __forceinline__ void bspmv_cta_by_output(int cta, int nrow, const int *__restrict__ IA,
+                                                    const int *__restrict__ JA, const TA *__restrict__ A,
+                                                    const double *__restrict__ x, double *__restrict__ y) {
+    const int64_t at = (int64_t)cta * kSpmvThreads + threadIdx.x;
+    const int r = (int)(at / 5), m = (int)(at - 5 * (int64_t)r);
+    if (r >= nrow) return;
+    double s0 = 0.0, s1 = 0.0;
+    int k = IA[r];
+    const int k1 = IA[r + 1];
+    for (; k + 1 < k1; k += 2) {
+        const TA *a = A + (int64_t)k * 25 + m * 5;
+        const double *xv = x + (int64_t)JA[k] * 5, *xw = x + (int64_t)JA[k + 1] * 5;
+        double av[10];
+#pragma unroll
+        for (int q = 0; q < 5; q++) {
+            av[q] = load_low(a + q);
+            av[5 + q] = load_low(a + 25 + q);
+        }
+#pragma unroll
+        for (int q = 0; q < 5; q++) {
+            s0 = fma(av[q], __ldg(xv + q), s0);
+            s1 = fma(av[5 + q], __ldg(xw + q), s1);
+        }
+    }
+    if (k < k1) {
+        const TA *a = A + (int64_t)k * 25 + m * 5;
+        const double *xv = x + (int64_t)JA[k] * 5;
+#pragma unroll
+        for (int q = 0; q < 5; q++) s0 = fma(load_low(a + q), __ldg(xv + q), s0);
+    }
+    y[(int64_t)r * 5 + m] = s0 + s1;
+}
+
+template <typename TA, bool BY_OUTPUT>
 __global__ void __launch_bounds__(kSpmvThreads) k_bspmv(int nrow, const int *__restrict__ IA, const int *__restrict__ JA,
                                                         const TA *__restrict__ A, const double *__restrict__ x,
                                                         double *__restrict__ y) {
-    bspmv_cta<TA>((int)blockIdx.x, nrow, IA, JA, A, x, y);
+    if constexpr (BY_OUTPUT) bspmv_cta_by_output<TA>((int)blockIdx.x, nrow, IA, JA, A, x, y);
+    else bspmv_cta<TA>((int)blockIdx.x, nrow, IA, JA, A, x, y);
+}
+
+// Whether a lane forms an output instead of a column's part: rows so short that
+// the columns' sums at the end and the first round of ids cost more than they
+// save.  Column / output, cold L2, FP32 / FP64 / BF16: 5 blocks per row (a plane of
+// 1000^2 rows) 150 / 219 / 145 and 129 / 195 / 115 us; 6 (300 x 300 x 2) 43 / 57 / 37
+// and 43 / 59 / 33; 7 (hexahedra, 90^3) 131 / 193 / 121 and 133 / 195 / 115; 14 (tets,
+// 70^3) 123 / 184 / 115 and 150 / 208 / 139.  BF16 matrices that stay in L2 gain from
+// the columns at 7 already (48^3: 22.4 and 24.5 us).  Boxes of tets, as the
+// serving loop solves them, lie above both lines: 5.75 blocks per row and, where
+// a BF16 matrix is that large, 7.9 and more.
+static bool spmv_by_output(int64_t nnzb, int64_t nrow, int prec) {
+    return 2 * nnzb <= 11 * nrow || (prec == CFD_PREC_BF16 && 2 * nnzb <= 15 * nrow && nnzb * 50 > ((int64_t)126 << 20));
 }
 
 // Several requests' SpMVs in one launch (the serving loop's fused SpMV): CTA
 // b belongs to the job whose [block_begin, next block_begin) holds it, and
-// computes that job's rows exactly as k_bspmv's CTA b - block_begin would.
+// computes that job's rows exactly as k_bspmv's CTA b - block_begin would (a
+// served box's rows are never short enough for a lane per output).
 template <typename TA>
 __global__ void __launch_bounds__(kSpmvThreads) k_bspmv_batch(const __grid_constant__ SpmvBatch B) {
     int j = 0;
@@ -812,7 +864,6 @@ static int precond_apply(cfd_ctx *c, const Precond &pc, const double *r, double 
 
 static int spmv(cfd_ctx *c, int prec, const double *x, double *y) {
     const int n = c->nnode;
-    const int g = spmv_blocks(n), b = kSpmvThreads;
     // the copies of this system: FP64 unless a64_valid says no, and a_precision;
     // what else is allocated belongs to an earlier system
     if (prec != c->a_precision) prec = CFD_PREC_FP64;
@@ -825,12 +876,17 @@ static int spmv(cfd_ctx *c, int prec, const double *x, double *y) {
         const SpmvJob job{n, c->IA.p, c->JA.p, A, x, y, 0};
         return c->batch_submit(c->batcher, c, kSpmvKey + prec, &job);
     }
+    const bool by_output = spmv_by_output(c->nnzb, n, prec);
+    const int g = by_output ? grid_for(5 * (int64_t)n, kSpmvThreads) : spmv_blocks(n);
+    auto run = [&](auto kern, auto *a) {
+        kern<<<g, kSpmvThreads, 0, c->stream>>>(n, c->IA.p, c->JA.p, a, x, y);
+    };
     if (prec == CFD_PREC_FP32)
-        k_bspmv<float><<<g, b, 0, c->stream>>>(n, c->IA.p, c->JA.p, static_cast<const float *>(A), x, y);
+        run(by_output ? k_bspmv<float, true> : k_bspmv<float, false>, static_cast<const float *>(A));
     else if (prec == CFD_PREC_BF16)
-        k_bspmv<uint16_t><<<g, b, 0, c->stream>>>(n, c->IA.p, c->JA.p, static_cast<const uint16_t *>(A), x, y);
+        run(by_output ? k_bspmv<uint16_t, true> : k_bspmv<uint16_t, false>, static_cast<const uint16_t *>(A));
     else
-        k_bspmv<double><<<g, b, 0, c->stream>>>(n, c->IA.p, c->JA.p, static_cast<const double *>(A), x, y);
+        run(by_output ? k_bspmv<double, true> : k_bspmv<double, false>, static_cast<const double *>(A));
     CFD_LAUNCH_CHECK();
     return CFD_OK;
 }
