@@ -645,11 +645,11 @@ __global__ void k_add_diss(int64_t n, const double *__restrict__ a, const double
 // us (58 / 61).  Bound by latency at three CTAs per SM (168 registers).  The
 // lanes stage their blocks in shared memory and the warp stores them one after
 // the other, 100 or 200 contiguous bytes each; a row's next block follows in
-// the next step, so the sectors they share fill in L2.  Eight of these stores
-// in flight suit BF16 blocks and Thornber's form (BF16, 66^3 cube: Thornber 534 /
-// 494 us with four / eight, Roe 413 / 397; 16: 515 and 406), four the others
-// (FP32 Roe 386 / 408); two matrices are stored by all 32 lanes (617 us, 642 with
-// a block per step).
+// the next step, so the sectors they share fill in L2.  BF16 blocks and
+// Thornber's form take this loop unrolled eight times (66^3 cube, BF16: Thornber
+// 531 -> 492 us, Roe 409 -> 394; 16 times 515 and 406), the others as the compiler
+// does (FP32 Roe 386 us; eight times 408, four 422, rolled 495); two matrices are
+// stored by all 32 lanes (617 us, 642 with a block per step).
 // The low-precision-only system sums the diagonal from the rounded blocks.
 // MODE: 0 Roe, 1 preconditioned Roe (CFD_FLUX_ROE_PRECOND), 2 Thornber (|A| of
 // the modified states).  RUP: the state's variables (f.rup).  HIGH / LOW: an
@@ -685,7 +685,6 @@ __global__ void __launch_bounds__(32 * JAC_WARPS, MODE == 1 ? 2 : 3) k_jacobian(
     int include_diss, Flow f, double *__restrict__ A64, TA *__restrict__ Alow, double *__restrict__ B) {
     f.rup = RUP ? 1 : 0;  // a compile-time constant below
     using TS = std::conditional_t<HIGH, double, TA>;  // staged blocks
-    constexpr int kUnroll = sizeof(TS) == 2 || MODE == 2 ? 8 : 4;  // of the stores
     __shared__ TS stage[JAC_WARPS][32][25];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x) / LANES, sub = lane % LANES;
@@ -746,13 +745,18 @@ __global__ void __launch_bounds__(32 * JAC_WARPS, MODE == 1 ? 2 : 3) k_jacobian(
             }
         } else {
             // a block per step, lane m element m
-#pragma unroll(kUnroll)
-            for (int b = 0; b < 32; b++) {
+            auto put_block = [&](int b) {
                 const int at = __shfl_sync(0xffffffffu, slot, b);
-                if (at < 0 || lane >= 25) continue;
+                if (at < 0 || lane >= 25) return;
                 const TS v = stage[w][b][lane];
                 if constexpr (HIGH) A64[(int64_t)at * 25 + lane] = v;
                 else Alow[(int64_t)at * 25 + lane] = v;
+            };
+            if constexpr (sizeof(TS) == 2 || MODE == 2) {
+#pragma unroll 8
+                for (int b = 0; b < 32; b++) put_block(b);
+            } else {
+                for (int b = 0; b < 32; b++) put_block(b);
             }
         }
         __syncwarp();
